@@ -53,10 +53,10 @@ int rha(double v) { return static_cast<int>(v >= 0 ? std::floor(v + 0.5) : -std:
 void gather_half(const float* G, const float* dA, const float* dR, float4* A, float2* B) {
   for (int j = 0; j < kSpecHalf; ++j) {
     const int py = j / kXhCols, sl = j - py * kXhCols;
-    const int kx = sl < 64 ? (sl >> 2) + 16 * (sl & 3) : 64;
+    const int kx = sl < 64 ? half_kx(sl) : 64;
     const int ky = 16 * (py & 7) + (py >> 3);
-    const int i1 = py * kTile + perm128(kx);
-    const int i2 = perm128((kTile - ky) & 127) * kTile + perm128((kTile - kx) & 127);
+    const int i1 = spectrum_pos(py, perm128(kx));
+    const int i2 = spectrum_pos(perm128((kTile - ky) & 127), perm128((kTile - kx) & 127));
     A[j] = make_float4(G[i1], G[i2], dA[i1], dR[i1]);
     const bool self = kx == 0 || kx == 64;
     B[j] = make_float2(self ? 0.f : dA[i2], self ? 0.f : dR[i2]);

@@ -226,7 +226,14 @@ __device__ __forceinline__ int perm128d(int k) { return 8 * (k & 15) + (k >> 4);
 // sum dG Re(conj(A) X), and Bh += (A G + conj(A G)(-k))/2.  The
 // per-orientation coefficients G(+-k), dGa, dGr come pre-gathered in the
 // half layout (ScaleDev::bwA, bwB).
-constexpr int kGaborBwdSmem = kSmemW + kSmemBh + kSmemTw + kSmemMaps + 16;
+// The work buffer keeps the unpadded layout: with the padded one (224 KB of
+// shared memory instead of 196) L1 no longer holds an orientation's block of
+// dL/dC (40 KB), and the backward of a 1333 x 1001 image took 4% longer.
+constexpr int kSmemBwW = kTile * kTile * 8;
+constexpr int kGaborBwdSmem = kSmemBwW + kSmemBh + kSmemTw + kSmemMaps + 16;
+static_assert(RotLayout::kHalf * 8 + kTile * RawWindow<true>::kPitch * 4 <= kSmemBwW + kSmemBh,
+              "the float window is staged behind the packed rows, over the accumulator");
+__device__ __forceinline__ int bwidx(int y, int p) { return RotLayout::at(y, p); }
 
 // Prefetch (into L2, or into this SM's L1) of the block of dL/dC that the
 // magnitude pass of one orientation reads: rows [R0, R0 + rows), columns
@@ -253,12 +260,11 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
   extern __shared__ float4 smem4b[];
   char* base = reinterpret_cast<char*>(smem4b);
   float2* W = reinterpret_cast<float2*>(base);
-  float2* Bh = reinterpret_cast<float2*>(base + kSmemW);
-  float2* tw = reinterpret_cast<float2*>(base + kSmemW + kSmemBh);
-  short* rmap = reinterpret_cast<short*>(base + kSmemW + kSmemBh + kSmemTw);
+  float2* Bh = reinterpret_cast<float2*>(base + kSmemBwW);
+  float2* tw = reinterpret_cast<float2*>(base + kSmemBwW + kSmemBh);
+  short* rmap = reinterpret_cast<short*>(base + kSmemBwW + kSmemBh + kSmemTw);
   short* cmap = rmap + kTile;
-  uint32_t* tmemSlot = reinterpret_cast<uint32_t*>(base + kSmemW + kSmemBh + kSmemTw + kSmemMaps);
-  float2* Xh64 = W + 64 * kTile;   // forward transform only
+  uint32_t* tmemSlot = reinterpret_cast<uint32_t*>(base + kSmemBwW + kSmemBh + kSmemTw + kSmemMaps);
   float2* Nyq = Bh;                // forward transform only (Bh is cleared after it)
   float2* __restrict__ Xs = xscratch + (size_t)blockIdx.x * kSpecHalf;
   const int t = threadIdx.x;
@@ -271,15 +277,7 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
   __syncthreads();
   tmem_fence_after();
   const uint32_t tlane = *tmemSlot + ((uint32_t)((t >> 5) & 3) << 21);
-  // column p of the full spectrum in the Hermitian half (as the forward)
-  const int pI1 = t & 127, h = t >> 7;
-  const int pa = pI1 >> 3, pb = pI1 & 7;
-  const bool pNyq = pb == 4 && pa == 0;
-  const bool pConj = pb >= 4 && !pNyq;
-  const int pSlot = pb < 4 ? 4 * pa + pb : (pNyq ? 64 : (pa > 0 ? 4 * (16 - pa) + (7 - pb) : 8 - pb));
-  const float pSign = pConj ? -1.f : 1.f;
-  const float2* pSrc = pNyq ? Nyq : Xh64 + pSlot;
-  const int pStride = pNyq ? 1 : 64;
+  const int h = t >> 7, pcol = RotLayout::col(t & 127);   // row group, this lane's column
   double accA = 0.0, accR = 0.0;
   for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
     const TileWork item = work[w];
@@ -288,23 +286,12 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
     const int ty = item.tile / sd->tilesX, tx = item.tile - ty * sd->tilesX;
     const int R0 = ty * V, C0 = tx * V;
     __syncthreads();   // previous tile finished with every buffer
-    tile_forward_spectrum<true>(sd, R0, C0, W, Xh64, Nyq, tw, rmap, cmap, t);
-#pragma unroll 1
-    for (int q = 0; q < 4; ++q) {
-      const int k2 = h + 4 * q;
-      float2 x[8];
-#pragma unroll
-      for (int k1 = 0; k1 < 8; ++k1) {
-        const int row = pConj ? (k2 > 0 ? 8 * (16 - k2) + (7 - k1) : (8 - k1) & 7) : 8 * k2 + k1;
-        x[k1] = pSrc[row * pStride];
-        x[k1].y *= pSign;
-      }
-      tmem_store8(tlane + 16 * k2, x);
-    }
-    for (int j = t; j < kSpecHalf; j += kTileThreads) {
-      const int r = j / kXhCols, sl = j - r * kXhCols;
-      Xs[j] = *xh_ptr(Xh64, Nyq, r, sl);
-    }
+    if (t < kTile) rmap[t] = (short)window_src(R0 - kX, t, sd->fftH, sd->dataH, kX);
+    else if (t < 2 * kTile) cmap[t - kTile] = (short)window_src(C0 - kX, t - kTile, sd->fftW, sd->dataW, kX);
+    float* raw = reinterpret_cast<float*>(W + RotLayout::kHalf);
+    raw_window_copy<true>(sd, R0, C0, raw, 0, 0, t);
+    __syncthreads();
+    tile_forward_spectrum<true, true, RotLayout>(raw, W, Nyq, tw, tlane, Xs, t, [] {});
     tmem_fence_before();
     __syncthreads();   // the Hermitian half in W / Bh is dead from here
     tmem_fence_after();
@@ -324,12 +311,14 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
         const int k2 = h + 4 * q;
         float2 v[8];
         tmem_load8(tlane + 16 * k2, v);
-        const float* __restrict__ Gq = Go + (size_t)(8 * k2) * kTile + pI1;
+        const float4* Ga = reinterpret_cast<const float4*>(Go) + gpos(8 * k2, glane(pcol)) / 4;
+        const float4 ga0 = __ldg(Ga), ga1 = __ldg(Ga + kTile);
+        const float ga[8] = {ga0.x, ga0.y, ga0.z, ga0.w, ga1.x, ga1.y, ga1.z, ga1.w};
         float2 twr[8];   // read before the TMEM stores (compiler barriers for shared loads)
 #pragma unroll
         for (int n1 = 1; n1 < 8; ++n1) twr[n1] = tw[n1 * 17 + k2];
 #pragma unroll
-        for (int k1 = 0; k1 < 8; ++k1) v[k1] = c_scale(v[k1], __ldg(Gq + k1 * kTile));
+        for (int k1 = 0; k1 < 8; ++k1) v[k1] = c_scale(v[k1], ga[k1]);
         dft8<true>(v);
 #pragma unroll
         for (int n1 = 0; n1 < 8; ++n1)
@@ -346,14 +335,14 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
 #pragma unroll
       for (int it = 0; it < 2; ++it) {
         const int j = t + it * kTileThreads;
-        const int p = j & 127, n1 = j >> 7;
+        const int p = pcol, n1 = j >> 7;
         float2 v[16];
         tmem_load16(tlane + kTmemY + 32 * n1, v);
         dft16<true>(v);
 #pragma unroll
         for (int n2 = 0; n2 < 16; ++n2) {
           const int y = n1 + 8 * n2;
-          W[widx(y, p)] = (y >= kX && y < kX + V) ? v[n2] : make_float2(0.f, 0.f);
+          W[bwidx(y, p)] = (y >= kX && y < kX + V) ? v[n2] : make_float2(0.f, 0.f);
         }
       }
       tmem_fence_before();
@@ -370,10 +359,10 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
           const int y = kX + (j >> 4);
           float2 v[8];
 #pragma unroll
-          for (int k1 = 0; k1 < 8; ++k1) v[k1] = W[widx(y, 8 * k2 + k1)];
+          for (int k1 = 0; k1 < 8; ++k1) v[k1] = W[bwidx(y, 8 * k2 + k1)];
           dft8<true>(v);
 #pragma unroll
-          for (int n1 = 0; n1 < 8; ++n1) W[widx(y, 8 * k2 + n1)] = n1 ? c_mulc(v[n1], twr[n1]) : v[0];
+          for (int n1 = 0; n1 < 8; ++n1) W[bwidx(y, 8 * k2 + n1)] = n1 ? c_mulc(v[n1], twr[n1]) : v[0];
         }
       }
       __syncthreads();
@@ -398,7 +387,7 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
         }
         float2 v[16];
 #pragma unroll
-        for (int k2 = 0; k2 < 16; ++k2) v[k2] = W[widx(y, 8 * k2 + n1)];
+        for (int k2 = 0; k2 < 16; ++k2) v[k2] = W[bwidx(y, 8 * k2 + n1)];
         dft16<true>(v);
 #pragma unroll
         for (int n2 = 0; n2 < 16; ++n2) {
@@ -425,44 +414,44 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
 #pragma unroll
         for (int k2 = 0; k2 < 16; ++k2) twr[k2] = tw[n1 * 17 + k2];
 #pragma unroll
-        for (int k2 = 0; k2 < 16; ++k2) W[widx(y, n1 + 8 * k2)] = c_mul(v[k2], twr[k2]);
+        for (int k2 = 0; k2 < 16; ++k2) W[bwidx(y, n1 + 8 * k2)] = c_mul(v[k2], twr[k2]);
       }
       __syncthreads();
       for (int j = t; j < V * 16; j += kTileThreads) {
         const int y = kX + (j >> 4), k2 = j & 15;
         float2 v[8];
 #pragma unroll
-        for (int n1 = 0; n1 < 8; ++n1) v[n1] = W[widx(y, 8 * k2 + n1)];
+        for (int n1 = 0; n1 < 8; ++n1) v[n1] = W[bwidx(y, 8 * k2 + n1)];
         dft8<false>(v);
 #pragma unroll
-        for (int k1 = 0; k1 < 8; ++k1) W[widx(y, 8 * k2 + k1)] = v[k1];
+        for (int k1 = 0; k1 < 8; ++k1) W[bwidx(y, 8 * k2 + k1)] = v[k1];
       }
       __syncthreads();
 #pragma unroll
       for (int it = 0; it < 2; ++it) {
         const int j = t + it * kTileThreads;
-        const int p = j & 127, n1 = j >> 7;
+        const int p = pcol, n1 = j >> 7;
         float2 v[16];
 #pragma unroll
-        for (int m = 0; m < 16; ++m) v[m] = W[widx(n1 + 8 * m, p)];
+        for (int m = 0; m < 16; ++m) v[m] = W[bwidx(n1 + 8 * m, p)];
         dft16<false>(v);
         float2 twr[16];
 #pragma unroll
         for (int k2 = 0; k2 < 16; ++k2) twr[k2] = tw[n1 * 17 + k2];
 #pragma unroll
-        for (int k2 = 0; k2 < 16; ++k2) W[widx(n1 + 8 * k2, p)] = c_mul(v[k2], twr[k2]);
+        for (int k2 = 0; k2 < 16; ++k2) W[bwidx(n1 + 8 * k2, p)] = c_mul(v[k2], twr[k2]);
       }
       __syncthreads();
 #pragma unroll
       for (int it = 0; it < 4; ++it) {
         const int j = t + it * kTileThreads;
-        const int p = j & 127, k2 = j >> 7;
+        const int p = pcol, k2 = j >> 7;
         float2 v[8];
 #pragma unroll
-        for (int n1 = 0; n1 < 8; ++n1) v[n1] = W[widx(8 * k2 + n1, p)];
+        for (int n1 = 0; n1 < 8; ++n1) v[n1] = W[bwidx(8 * k2 + n1, p)];
         dft8<false>(v);
 #pragma unroll
-        for (int k1 = 0; k1 < 8; ++k1) W[widx(8 * k2 + k1, p)] = v[k1];
+        for (int k1 = 0; k1 < 8; ++k1) W[bwidx(8 * k2 + k1, p)] = v[k1];
       }
       __syncthreads();
       // Hermitian accumulation and the parameter dot products.  Entry j of
@@ -482,7 +471,7 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
           const float2 X = Xs[j];   // written by this CTA for this tile: a coherent load
           const int ky = 16 * (py & 7) + (py >> 3);
           const int npy = perm128d((kTile - ky) & 127);
-          const float2 A1 = W[wp], A2 = W[widx(npy, np)];
+          const float2 A1 = W[wp], A2 = W[bwidx(npy, np)];
           const float2 bb = Bh[j];
           Bh[j] = make_float2(fmaf(0.5f * c4.x, A1.x, fmaf(0.5f * c4.y, A2.x, bb.x)),
                               fmaf(0.5f * c4.x, A1.y, fmaf(-0.5f * c4.y, A2.y, bb.y)));
@@ -492,16 +481,15 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
           sr = fmaf(c4.w, re1, fmaf(c2.y, re2, sr));
         };
         // slots 0..63: thread t owns slot sl = t mod 64 and the rows
-        // py = t / 64 + 8 r (r = 0..15), so its column terms are fixed and
-        // widx(py, p) = 128 py + (phys(p) ^ 8 (py & 1)) with py & 1 fixed
+        // py = t / 64 + 8 r (r = 0..15), so its column terms are fixed
         // Four entries at a time: all their loads first, then the updates
         // (the entries' Bh words are distinct, but a store would otherwise
         // hold back the next entry's shared-memory loads).
         {
           const int sl = t & 63, pr = t >> 6;
-          const int kx = (sl >> 2) + 16 * (sl & 3);
+          const int kx = half_group(sl) + 16 * (sl & 3);
           const int p = perm128d(kx), np = perm128d((kTile - kx) & 127);
-          const int pp = phys(p) ^ ((pr & 1) << 3);
+          const int pp = bwidx(pr & 1, p) - (pr & 1) * kTile;
 #pragma unroll 1
           for (int r0 = 0; r0 < 16; r0 += 4) {
             float4 c4[4];
@@ -515,7 +503,7 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
               X[u] = Xs[j];
               const int ky = 16 * (py & 7) + (py >> 3);
               A1[u] = W[py * kTile + pp];
-              A2[u] = W[widx(perm128d((kTile - ky) & 127), np)];
+              A2[u] = W[bwidx(perm128d((kTile - ky) & 127), np)];
               bb[u] = Bh[j];
             }
 #pragma unroll
@@ -532,8 +520,9 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
         }
         // the Nyquist slot 64 (kx = 64): one row per thread of the first 128
         if (t < kTile) {
-          const int p = perm128d(64);
-          entry(t, 64, p, p, widx(t, p));
+          const int p = perm128d(64), sl = t & 63;
+          const int row = (t & 64) + 4 * half_group(sl) + (sl & 3);
+          entry(row, 64, p, p, bwidx(row, p));
         }
         accA += sa;
         accR += sr;
@@ -544,17 +533,16 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
     __syncthreads();
     // one inverse transform of the Hermitian sum: Re -> window gradient,
     // scattered to the float level through the padded-torus index maps.
-    // Column p = t & 127 of the full spectrum is read from the half Bh
+    // This lane's column of the full spectrum is read from the half Bh
     // without a branch (conj(Bh(-k)) for kx > 64).
-    const int pa = (t & 127) >> 3, pb = t & 7;
-    const bool pNyq = pb == 4 && pa == 0;
-    const bool pConj = pb >= 4 && !pNyq;
-    const int pSlot = pb < 4 ? 4 * pa + pb : (pNyq ? 64 : (pa > 0 ? 4 * (16 - pa) + (7 - pb) : 8 - pb));
+    const HalfColumn hc(pcol);
+    const bool pConj = hc.conj;
+    const int pSlot = hc.slot;
     const float pSign = pConj ? -1.f : 1.f;
 #pragma unroll
     for (int it = 0; it < 4; ++it) {
       const int j = t + it * kTileThreads;
-      const int p = j & 127, k2 = j >> 7;
+      const int p = pcol, k2 = j >> 7;
       float2 v[8];
 #pragma unroll
       for (int k1 = 0; k1 < 8; ++k1) {
@@ -564,19 +552,19 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
       }
       dft8<true>(v);
 #pragma unroll
-      for (int n1 = 0; n1 < 8; ++n1) W[widx(8 * k2 + n1, p)] = c_mulc(v[n1], tw[n1 * 17 + k2]);
+      for (int n1 = 0; n1 < 8; ++n1) W[bwidx(8 * k2 + n1, p)] = c_mulc(v[n1], tw[n1 * 17 + k2]);
     }
     __syncthreads();
 #pragma unroll
     for (int it = 0; it < 2; ++it) {
       const int j = t + it * kTileThreads;
-      const int p = j & 127, n1 = j >> 7;
+      const int p = pcol, n1 = j >> 7;
       float2 v[16];
 #pragma unroll
-      for (int k2 = 0; k2 < 16; ++k2) v[k2] = W[widx(8 * k2 + n1, p)];
+      for (int k2 = 0; k2 < 16; ++k2) v[k2] = W[bwidx(8 * k2 + n1, p)];
       dft16<true>(v);
 #pragma unroll
-      for (int n2 = 0; n2 < 16; ++n2) W[widx(n1 + 8 * n2, p)] = v[n2];
+      for (int n2 = 0; n2 < 16; ++n2) W[bwidx(n1 + 8 * n2, p)] = v[n2];
     }
     __syncthreads();
 #pragma unroll
@@ -585,10 +573,10 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
       const int y = j >> 4, k2 = j & 15;
       float2 v[8];
 #pragma unroll
-      for (int k1 = 0; k1 < 8; ++k1) v[k1] = W[widx(y, 8 * k2 + k1)];
+      for (int k1 = 0; k1 < 8; ++k1) v[k1] = W[bwidx(y, 8 * k2 + k1)];
       dft8<true>(v);
 #pragma unroll
-      for (int n1 = 0; n1 < 8; ++n1) W[widx(y, 8 * k2 + n1)] = c_mulc(v[n1], tw[n1 * 17 + k2]);
+      for (int n1 = 0; n1 < 8; ++n1) W[bwidx(y, 8 * k2 + n1)] = c_mulc(v[n1], tw[n1 * 17 + k2]);
     }
     __syncthreads();
     float* __restrict__ gl = sd->gLvl;
@@ -599,7 +587,7 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
       const int y = j >> 3, n1 = j & 7;
       float2 v[16];
 #pragma unroll
-      for (int k2 = 0; k2 < 16; ++k2) v[k2] = W[widx(y, 8 * k2 + n1)];
+      for (int k2 = 0; k2 < 16; ++k2) v[k2] = W[bwidx(y, 8 * k2 + n1)];
       dft16<true>(v);
       float* row = gl + (size_t)rmap[y] * gp;
 #pragma unroll

@@ -132,8 +132,10 @@ bool build_scales(int width, int height, const std::vector<float>& lambdas_in,
 //   G(k) = Re sum_d q(d) exp(-2 pi i k.d / 128) / 128^2
 // The even taps are point-symmetric and the odd taps antisymmetric, so the
 // imaginary part is only the float rounding of the taps and is dropped.
-// Stored at [o][perm128(ky)][perm128(kx)], the digit-permuted order in which
-// the kernel's forward transform leaves the image spectrum.
+// Entry (ky, kx) is stored at spectrum_pos(perm128(ky), perm128(kx)) of
+// orientation o's 128 x 128 block: the digit-permuted order in which the
+// kernel's forward transform leaves the image spectrum, columns in the order of
+// the tensor-memory lanes that hold them, rows in groups of four.
 void tile_spectrum(const std::vector<float>* even, const std::vector<float>* odd, int kW, int kX,
                    std::vector<float>& out) {
   const int T = kTile, n = kW, h = kX;
@@ -167,7 +169,7 @@ void tile_spectrum(const std::vector<float>* even, const std::vector<float>* odd
           const int m = ((ky * (row - h)) % T + T) % T;
           re += rre[row * T + kx] * cs[m] + rim[row * T + kx] * sn[m];
         }
-        out[(static_cast<size_t>(o) * T + perm128(ky)) * T + perm128(kx)] =
+        out[static_cast<size_t>(o) * T * T + spectrum_pos(perm128(ky), perm128(kx))] =
             static_cast<float>(re / (double(T) * T));
       }
     }

@@ -37,7 +37,7 @@ struct ScaleDev {
   // level image (uint8, full pyrDown size lvlW x lvlH)
   const uint8_t* lvl;
   int lvlPitch, lvlW, lvlH;
-  // real tile spectra, kNumOri x kTile x kTile floats in (py, px) order
+  // real tile spectra, kNumOri x kTile x kTile floats (see spectrum_pos)
   const float* G;
   // complex-cell maps: kNumOri maps, each cRows x cPitch floats
   float* C;
@@ -78,6 +78,7 @@ struct ScaleDev {
   unsigned int* bits;     // ReLU states, 4 bits per orientation, dataH x dPitch
   const float4* bwA;      // per orientation, kSpecHalf entries {G(k), G(-k), dGa(k), dGr(k)}
   const float2* bwB;      //   {dGa(-k), dGr(-k)}; dG* = spectra of d taps / d alpha, d rho
+  int pad[2];             // to a multiple of 16 bytes: the tile kernel copies records as 16-byte words
 };
 
 // Stencil offset sets of the two level wavelengths the default bank uses
@@ -98,7 +99,7 @@ constexpr int kOffsetSets[kNumOffsetSets][6][8] = BIMP_OFFSET_SETS;
 
 // One unit of tiled-FFT work: orientations [oBegin, oEnd) of tile `tile` of
 // descriptor `entry`.  oBegin == oEnd is an empty slot of a padded plan.
-struct TileWork {
+struct alignas(16) TileWork {
   int entry;
   int tile;
   int oBegin = 0;
@@ -132,5 +133,14 @@ int configure_device(int dev);
 
 // Position of natural frequency k in the digit-permuted 128-point layout.
 inline int perm128(int k) { return 8 * (k & 15) + (k >> 4); }
+// Where a stored Gabor spectrum keeps permuted row py, permuted column p: the
+// column's tensor-memory lane (groups j and j + 8 of eight columns share a half
+// warp), four rows of a column side by side.
+inline int spectrum_pos(int py, int p) {
+  const int lane = 16 * ((p >> 3) & 7) + 8 * (p >> 6) + (p & 7);
+  return ((py >> 2) * kTile + lane) * 4 + (py & 3);
+}
+// Column kx (0..63) of slot `slot` (0..63) of a Hermitian half spectrum.
+inline int half_kx(int slot) { return (slot >> 4) + 4 * ((slot >> 2) & 3) + 16 * (slot & 3); }
 
 }  // namespace bimp_b200

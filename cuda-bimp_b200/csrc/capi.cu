@@ -165,31 +165,27 @@ struct Engine {
   // orientation) pairs, tile by tile in plan order, are cut into at most
   // `grid` contiguous runs of about equal cost; a run becomes one work item
   // per tile it touches (a tile cut between two CTAs is transformed forward by
-  // both).  Costs come from the kernel's measured phase times (cycles between
-  // its CTA barriers at 1080p, in units of one orientation of a V = 100
-  // tile): per orientation, the product and inverse y-passes on all 128
-  // columns 0.414, each round of the first inverse x-pass (16 items per valid
-  // row inside the map over 512 threads) 0.0565, each round of the second
-  // (8 items per row) 0.18, of which
-  // the magnitudes and stores are 0.42 and scale with the share of the
-  // tile's outputs inside the map; an item's forward transform and spectrum
-  // store 1.35.  The smallest run bound that fits in `grid` runs is found by
-  // bisection.  Item k of CTA b is
+  // both).  Costs are a fit to the kernel's measured item times (1080p, cycles;
+  // residual 1.7 k of about 90 k an item): 14.5 k for an item's forward
+  // transform, and per orientation 5.0 k + 0.77 k for each block of four rows
+  // (of the rows inside the map) on the scheduler with most of them; in units
+  // of an orientation of a V = 100 tile.  The weights before the x-passes went
+  // warp by warp left 3840 x 2160 at 946 us, these 859.  The smallest run bound
+  // that fits in `grid` runs is found by bisection.  Item k of CTA b is
   // placed at index k * grid + b (the kernel strides its work list by the
   // grid); CTAs with fewer items get empty ones.  *usedGrid receives the
   // number of CTAs with work.
   static std::vector<TileWork> split_plan(const std::vector<TileWork>& tiles, const std::vector<ScaleDev>& sds,
                                           int grid, int* usedGrid) {
-    const double kFwd = 1.35;
+    const double kFwd = 1.4;
     std::vector<double> ori(tiles.size());
     double total = 0.0, worst = 0.0;
     for (size_t i = 0; i < tiles.size(); ++i) {
       const ScaleDev& d = sds[tiles[i].entry];
-      const int ty = tiles[i].tile / d.tilesX, tx = tiles[i].tile - ty * d.tilesX;
+      const int ty = tiles[i].tile / d.tilesX;
       const int vr = std::min(d.V, d.cRows - ty * d.V);   // valid rows inside the map (the x-passes' rows)
-      const double inside = (double)vr * std::min(d.V, d.cCols - tx * d.V) / ((double)d.V * d.V);
-      const int r3 = (16 * vr + kTileThreads - 1) / kTileThreads, r4 = (8 * vr + kTileThreads - 1) / kTileThreads;
-      ori[i] = 0.414 + 0.0565 * r3 + 0.18 * r4 * (0.58 + 0.42 * inside);
+      const int blocks = ((vr + 3) / 4 + 3) / 4;   // four-row blocks of the busiest scheduler
+      ori[i] = 0.481 + 0.0741 * blocks;
       total += kNumOri * ori[i] + kFwd;
       worst = std::max(worst, ori[i] + kFwd);
     }

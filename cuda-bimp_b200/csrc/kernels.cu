@@ -229,9 +229,12 @@ __global__ void __launch_bounds__(kPyrThreads) k_pyr_down(const PyrJob* __restri
 // ---------------------------------------------------------------------------
 __constant__ float2 c_w128[kTile];   // exp(-2 pi i k / 128)
 
+// a mod m for an a within a few m of [0, m) (a tile window's positions on its
+// torus): no division.
 __device__ __forceinline__ int pmod(int a, int m) {
-  const int r = a % m;
-  return r < 0 ? r + m : r;
+  while (a < 0) a += m;
+  while (a >= m) a -= m;
+  return a;
 }
 
 // Source row/col of padded-torus index t (convolutionFFT2D.cuh:56-85):
@@ -588,13 +591,6 @@ __device__ __forceinline__ void stencil_stage_tma(const void* cMap, int x0, int 
       : "memory");
 }
 
-__device__ __forceinline__ void mbar_init_count(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-
 template <int MODE>
 __global__ void __launch_bounds__(kStThreads, kStCtasPerSm)
 k_stencil(const ScaleDev* __restrict__ sds, const int2* __restrict__ work, int nwork,
@@ -612,8 +608,8 @@ k_stencil(const ScaleDev* __restrict__ sds, const int2* __restrict__ work, int n
   const uint32_t full0 = smem_u32(&s_full[0]), empty0 = smem_u32(&s_empty[0]);
   if (t == 0) {
     for (int i = 0; i < kStBufs; ++i) {
-      mbar_init_count(full0 + 8 * i, 1);
-      mbar_init_count(empty0 + 8 * i, kStConsumers / 32);
+      mbar_init(full0 + 8 * i, 1);
+      mbar_init(empty0 + 8 * i, kStConsumers / 32);
     }
     fence_mbar_init();
   }
