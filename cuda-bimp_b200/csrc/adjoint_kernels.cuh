@@ -206,53 +206,54 @@ k_stencil_bwd(const ScaleDev* __restrict__ sds, const int2* __restrict__ work) {
 // where z / |z| is the direction of rounding noise.  The floor is an
 // absolute value for images on the [0, 1] scale.
 constexpr float kMagFloor = 3.0e-5f;
-constexpr int kSmemBh = kSmemXh;   // Hermitian half of the accumulated spectrum
-
 // Position of natural frequency k in the digit-permuted order of the 8x16
 // transforms (the order of G and of the saved spectra).
 __device__ __forceinline__ int perm128d(int k) { return 8 * (k & 15) + (k >> 4); }
 
-// Persistent CTAs walk the tiles (one CTA per SM: 196 KB of shared memory
-// and all 512 TMEM columns).  The window gradient is linear in the
-// per-orientation spectra, Re IFFT(sum_o A_o G_o), so the products are summed
-// in the frequency domain (Hermitian half, Bh) and ONE inverse transform per
-// tile replaces one per orientation.  Nothing of the forward's responses is
-// stored: per tile the image spectrum X is recomputed from the float level
-// (the forward's transform: full spectrum into TMEM, Hermitian half into this
-// CTA's slot of `xscratch`), and per orientation e + i o is recomputed on the
-// valid outputs by the forward's inverse passes (G read from L2 instead of
-// staged); then a = dL/dC * z/|z| (0 where |z| <= kMagFloor or outside the
-// valid outputs), A = FFT(a), the alpha/rho dot products
-// sum dG Re(conj(A) X), and Bh += (A G + conj(A G)(-k))/2.  The
-// per-orientation coefficients G(+-k), dGa, dGr come pre-gathered in the
-// half layout (ScaleDev::bwA, bwB).
-// The work buffer keeps the unpadded layout: with the padded one (224 KB of
-// shared memory instead of 196) L1 no longer holds an orientation's block of
-// dL/dC (40 KB), and the backward of a 1333 x 1001 image took 4% longer.
-constexpr int kSmemBwW = kTile * kTile * 8;
-constexpr int kGaborBwdSmem = kSmemBwW + kSmemBh + kSmemTw + kSmemMaps + 16;
-static_assert(RotLayout::kHalf * 8 + kTile * RawWindow<true>::kPitch * 4 <= kSmemBwW + kSmemBh,
-              "the float window is staged behind the packed rows, over the accumulator");
-__device__ __forceinline__ int bwidx(int y, int p) { return RotLayout::at(y, p); }
+// Persistent CTAs walk the work items, each a tile and a run of its
+// orientations (one CTA per SM: 223 KB of shared memory and all 512 TMEM
+// columns).  The window gradient is linear in the per-orientation spectra,
+// Re IFFT(sum_o A_o G_o), so the products are summed in the frequency domain
+// (Hermitian half, Bh) and ONE inverse transform per item replaces one per
+// orientation.  Nothing of the forward's responses is stored: per item the
+// image spectrum X is recomputed from the float level (the forward's
+// transform: full spectrum into TMEM, Hermitian half into this CTA's slot of
+// `xscratch`), and per orientation e + i o is recomputed on the valid outputs
+// by the forward's inverse passes (G read from L2 instead of staged); then
+// a = dL/dC * z/|z| (0 where |z| <= kMagFloor or outside the valid outputs),
+// A = FFT(a), the alpha/rho dot products sum dG Re(conj(A) X), and
+// Bh += (A G + conj(A G)(-k))/2.  The per-orientation coefficients G(+-k),
+// dGa, dGr come pre-gathered in the half layout (ScaleDev::bwA, bwB).
+//
+// The x-passes of both directions run on the same rows, so a warp takes
+// blocks of four valid rows through all of them (inverse 8 and 16, magnitude,
+// forward 16 and 8) with no CTA barrier, its dL/dC values loaded before the
+// first; the y-passes meet at barriers of the four warps of a lane block.  Three
+// CTA barriers an orientation are left of seven.
+constexpr int kBwRaw = kTile * RawWindow<true>::kPitch * 4;   // staged float window, over Bh
+constexpr int kSmemBwBh = kBwRaw > kSmemXh ? kBwRaw : kSmemXh;
+constexpr int kGaborBwdSmem = kSmemW + kSmemBwBh + kSmemTw + kSmemMaps + 32;
+static_assert(kGaborBwdSmem <= 232448, "tile backward exceeds the 227 KB shared-memory limit");
 
-// Prefetch (into L2, or into this SM's L1) of the block of dL/dC that the
-// magnitude pass of one orientation reads: rows [R0, R0 + rows), columns
-// [x0, x1) of a map with row pitch `pitch` floats (rows start on 128-byte
-// lines).  One 128-byte line per thread and step; addresses stay inside the
-// map.  The loads come after three transform passes, so the lines are in
-// place by then instead of each load waiting on device memory.
-template <bool L1>
+// Prefetch into L2 of the block of dL/dC that one orientation's magnitude pass
+// reads: rows [R0, R0 + rows), columns [x0, x1) of a map with row pitch `pitch`
+// floats (rows start on 128-byte lines).  One 128-byte line per thread and
+// step; addresses stay inside the map.
 __device__ __forceinline__ void prefetch_block(const float* base, int pitch, int R0, int rows, int x0, int x1, int t) {
   if (rows <= 0 || x1 <= x0) return;
   const int l0 = x0 >> 5, nl = ((x1 - 1) >> 5) - l0 + 1;   // 32 floats per line
   for (int i = t; i < rows * nl; i += kTileThreads) {
     const int r = i / nl, l = l0 + (i - r * nl);
-    const float* a = base + (size_t)(R0 + r) * pitch + 32 * l;
-    if constexpr (L1) asm volatile("prefetch.global.L1 [%0];" ::"l"(a));
-    else asm volatile("prefetch.global.L2 [%0];" ::"l"(a));
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(base + (size_t)(R0 + r) * pitch + 32 * l));
   }
 }
-static_assert(kGaborBwdSmem <= 232448, "tile backward exceeds the 227 KB shared-memory limit");
+
+// The coefficients and image spectrum of four entries of the accumulation.
+struct BwEntries {
+  float4 c4[4];   // G(k), G(-k), dGa(k), dGr(k)
+  float2 c2[4];   // dGa(-k), dGr(-k)
+  float2 X[4];
+};
 
 __global__ void __launch_bounds__(kTileThreads, 1)
 k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__ work, int nwork,
@@ -260,340 +261,368 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
   extern __shared__ float4 smem4b[];
   char* base = reinterpret_cast<char*>(smem4b);
   float2* W = reinterpret_cast<float2*>(base);
-  float2* Bh = reinterpret_cast<float2*>(base + kSmemBwW);
-  float2* tw = reinterpret_cast<float2*>(base + kSmemBwW + kSmemBh);
-  short* rmap = reinterpret_cast<short*>(base + kSmemBwW + kSmemBh + kSmemTw);
+  float2* Bh = reinterpret_cast<float2*>(base + kSmemW);
+  float2* tw = reinterpret_cast<float2*>(base + kSmemW + kSmemBwBh);
+  short* rmap = reinterpret_cast<short*>(base + kSmemW + kSmemBwBh + kSmemTw);
   short* cmap = rmap + kTile;
-  uint32_t* tmemSlot = reinterpret_cast<uint32_t*>(base + kSmemBwW + kSmemBh + kSmemTw + kSmemMaps);
-  float2* Nyq = Bh;                // forward transform only (Bh is cleared after it)
+  uint64_t* bars = reinterpret_cast<uint64_t*>(base + kSmemW + kSmemBwBh + kSmemTw + kSmemMaps);
+  uint32_t* tmemSlot = reinterpret_cast<uint32_t*>(bars + 2);
+  const uint32_t barW = smem_u32(bars);
+  float2* Nyq = Bh;                                 // forward transform only (Bh is cleared after it)
+  float* rawBuf = reinterpret_cast<float*>(Bh);     // the staged window, before Bh and Nyq
   float2* __restrict__ Xs = xscratch + (size_t)blockIdx.x * kSpecHalf;
   const int t = threadIdx.x;
   if (t < 8 * 17) {
     const int n1 = t / 17, k2 = t % 17;
     tw[t] = k2 < 16 ? c_w128[(n1 * k2) & 127] : make_float2(0.f, 0.f);
   }
+  if (t == 0) {
+    mbar_init(barW, kTileThreads / 32);
+    fence_mbar_init();
+  }
   if ((t >> 5) == 0) tmem_alloc_warp(smem_u32(tmemSlot));
   tmem_fence_before();
   __syncthreads();
   tmem_fence_after();
   const uint32_t tlane = *tmemSlot + ((uint32_t)((t >> 5) & 3) << 21);
-  const int h = t >> 7, pcol = RotLayout::col(t & 127);   // row group, this lane's column
+  const int h = t >> 7, pcol = PadLayout::col(t & 127);   // row group, this lane's column
+  const int warp = t >> 5, quad = warp & 3, lane = t & 31;
+  uint32_t phW = 0;
   double accA = 0.0, accR = 0.0;
   for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
     const TileWork item = work[w];
+    const int oB = item.oBegin, oE = item.oEnd;
+    if (oB >= oE) break;   // the empty slots of a padded plan follow a CTA's last item
     const ScaleDev* sd = sds + item.entry;
     const int kX = sd->kX, V = sd->V;
     const int ty = item.tile / sd->tilesX, tx = item.tile - ty * sd->tilesX;
     const int R0 = ty * V, C0 = tx * V;
+    // rows and columns of the tile's valid outputs inside the map
+    const int Vr = min(V, sd->cRows - R0), xHi = min(kX + V, sd->cCols - C0 + kX);
+    const int cPitch = sd->cPitch;
     __syncthreads();   // previous tile finished with every buffer
+    raw_chunks_load<true>(sd, R0, C0, rawBuf, t);
     if (t < kTile) rmap[t] = (short)window_src(R0 - kX, t, sd->fftH, sd->dataH, kX);
     else if (t < 2 * kTile) cmap[t - kTile] = (short)window_src(C0 - kX, t - kTile, sd->fftW, sd->dataW, kX);
-    float* raw = reinterpret_cast<float*>(W + RotLayout::kHalf);
-    raw_window_copy<true>(sd, R0, C0, raw, 0, 0, t);
+    float* raw = rawBuf + ((C0 - kX) & 3);
+    {
+      const WindowSpan<true> span(sd, C0);
+      if (!span.all()) raw_window_copy<true>(sd, R0, C0, raw, span.iA, span.iB, t);
+    }
+    prefetch_block(sd->gC + (size_t)oB * sd->cStride, cPitch, R0, Vr, C0, C0 + xHi - kX, t);
+    cp_async_wait();
     __syncthreads();
-    tile_forward_spectrum<true, true, RotLayout>(raw, W, Nyq, tw, tlane, Xs, t, [] {});
+    tile_forward_spectrum<true, true, PadLayout>(raw, W, Nyq, tw, tlane, Xs, t, [] {});
     tmem_fence_before();
-    __syncthreads();   // the Hermitian half in W / Bh is dead from here
+    __syncthreads();   // the half spectrum in W / Bh is dead from here; X complete in TMEM and Xs
     tmem_fence_after();
     for (int j = t; j < kTile * kXhCols; j += kTileThreads) Bh[j] = make_float2(0.f, 0.f);
-    const int cRows = sd->cRows, cCols = sd->cCols, cPitch = sd->cPitch;
-    const long long cStride = sd->cStride;
-    const int wrapW = sd->wrapW;
-    // this tile's block of every dL/dC map: rows and columns of its valid
-    // outputs inside the map
-    const int pfRows = min(V, cRows - R0), pfX1 = min(C0 + V, cCols);
-    for (int o = 0; o < kNumOri; ++o) {
-      const float* __restrict__ Go = sd->G + (size_t)o * kSpecFloats;
-      prefetch_block<false>(sd->gC + (size_t)o * cStride, cPitch, R0, pfRows, C0, pfX1, t);
+    // x-pass lanes keep column group n1 = t mod 8: bit n2 says whether output
+    // x = n1 + 8 n2 is valid and inside the map; bit n2 + 16 it of yMask the
+    // same of I2's row h + 4 it + 8 n2
+    unsigned int xMask = 0, yMask = 0;
+#pragma unroll
+    for (int n2 = 0; n2 < 16; ++n2) {
+      const int x = (t & 7) + 8 * n2, y = h + 8 * n2;
+      xMask |= (x >= kX && x < xHi ? 1u : 0u) << n2;
+      yMask |= (y >= kX && y < kX + Vr ? 1u : 0u) << n2 | (y + 4 >= kX && y + 4 < kX + Vr ? 0x10000u : 0u) << n2;
+    }
+    for (int o = oB; o < oE; ++o) {
       // I1: y-dim pass B' with the spectrum product X * G_o (TMEM in, TMEM out)
-#pragma unroll 1
-      for (int q = 0; q < 4; ++q) {
-        const int k2 = h + 4 * q;
-        float2 v[8];
-        tmem_load8(tlane + 16 * k2, v);
-        const float4* Ga = reinterpret_cast<const float4*>(Go) + gpos(8 * k2, glane(pcol)) / 4;
-        const float4 ga0 = __ldg(Ga), ga1 = __ldg(Ga + kTile);
-        const float ga[8] = {ga0.x, ga0.y, ga0.z, ga0.w, ga1.x, ga1.y, ga1.z, ga1.w};
-        float2 twr[8];   // read before the TMEM stores (compiler barriers for shared loads)
+      {
+        // all of the thread's G under way before its first use
+        const float4* Go = reinterpret_cast<const float4*>(sd->G + (size_t)o * kSpecFloats) + gpos(8 * h, t & 127) / 4;
+        float4 g0[4], g1[4];
 #pragma unroll
-        for (int n1 = 1; n1 < 8; ++n1) twr[n1] = tw[n1 * 17 + k2];
+        for (int q = 0; q < 4; ++q) {
+          g0[q] = __ldg(Go + 8 * q * kTile);
+          g1[q] = __ldg(Go + (8 * q + 1) * kTile);
+        }
 #pragma unroll
-        for (int k1 = 0; k1 < 8; ++k1) v[k1] = c_scale(v[k1], ga[k1]);
-        dft8<true>(v);
+        for (int q = 0; q < 4; ++q) {
+          const int k2 = h + 4 * q;
+          float2 v[8];
+          tmem_load8(tlane + 16 * k2, v);
+          const float ga[8] = {g0[q].x, g0[q].y, g0[q].z, g0[q].w, g1[q].x, g1[q].y, g1[q].z, g1[q].w};
+          float2 twr[8];
 #pragma unroll
-        for (int n1 = 0; n1 < 8; ++n1)
-          tmem_store1(tlane + kTmemY + 2 * (16 * n1 + k2), n1 ? c_mulc(v[n1], twr[n1]) : v[0]);
+          for (int n1 = 1; n1 < 8; ++n1) twr[n1] = tw[n1 * 17 + k2];
+#pragma unroll
+          for (int k1 = 0; k1 < 8; ++k1) v[k1] = c_scale(v[k1], ga[k1]);
+          dft8<true>(v);
+#pragma unroll
+          for (int n1 = 0; n1 < 8; ++n1)
+            tmem_store1(tlane + kTmemY + 2 * (16 * n1 + k2), n1 ? c_mulc(v[n1], twr[n1]) : v[0]);
+        }
       }
       tmem_wait_st();
       tmem_fence_before();
-      __syncthreads();   // the y-pass output is complete; no thread still reads W
+      named_barrier(1 + quad, kTileThreads / 4);   // the lane block's first y-pass is complete
       tmem_fence_after();
-      // (I2 and I3 use TMEM and shared memory only: L1 keeps the block)
-      prefetch_block<true>(sd->gC + (size_t)o * cStride, cPitch, R0, pfRows, C0, pfX1, t);
+      if (o > oB) {   // every warp is done with the previous orientation's accumulation
+        mbar_wait(barW, phW);
+        phW ^= 1u;
+        __syncwarp();
+      }
       // I2: y-dim pass A' -> natural y; rows outside the valid band are zero
       // (a is zero there, and the transform of a below reads every row)
 #pragma unroll
       for (int it = 0; it < 2; ++it) {
-        const int j = t + it * kTileThreads;
-        const int p = pcol, n1 = j >> 7;
+        const int n1 = h + 4 * it;
         float2 v[16];
         tmem_load16(tlane + kTmemY + 32 * n1, v);
         dft16<true>(v);
 #pragma unroll
         for (int n2 = 0; n2 < 16; ++n2) {
-          const int y = n1 + 8 * n2;
-          W[bwidx(y, p)] = (y >= kX && y < kX + V) ? v[n2] : make_float2(0.f, 0.f);
+          W[widx(n1 + 8 * n2, pcol)] = (yMask >> (n2 + 16 * it)) & 1u ? v[n2] : make_float2(0.f, 0.f);
         }
       }
       tmem_fence_before();
       __syncthreads();
       tmem_fence_after();
-      // I3: x-dim pass B' on the valid rows (a thread's k2 is fixed: its
-      // twiddles are read once, not behind each store)
+      if (o + 1 < oE)
+        prefetch_block(sd->gC + (size_t)(o + 1) * sd->cStride, cPitch, R0, Vr, C0, C0 + xHi - kX, t);
+      // The x-passes, four valid rows to a warp at a time: I3 (x-dim pass B');
+      // I4 (pass A': z = e + i o at the row's outputs x = n1 + 8 n2),
+      // a = dL/dC * z/|z| (|z| as the forward computed it) and the forward
+      // pass A of a on the same 16 elements, in registers; pass B.
       {
-        const int k2 = t & 15;
-        float2 twr[8];
+        const int k2 = lane & 15, n1 = lane & 7;
+        // dL/dC of output x = n1 + 8 n2 of the lane's row: src[8 n2]
+        const float* __restrict__ src = sd->gC + o * sd->cStride + (long long)(R0 + 4 * warp + (lane >> 3)) * cPitch +
+                                        (C0 - kX) + n1;
+        // fftW == dataW: window element (r + 1, 0) also carries the gradient
+        // of (r, dataW)
+        const bool wrapped = sd->wrapW && C0 == 0 && n1 == (kX & 7);
+#pragma unroll 1
+        for (int r0 = 4 * warp; r0 < Vr; r0 += 4 * (kTileThreads / 32), src += 4 * (kTileThreads / 32) * cPitch) {
+          const int r = r0 + (lane >> 3);
+          float gcv[16];
 #pragma unroll
-        for (int n1 = 1; n1 < 8; ++n1) twr[n1] = tw[n1 * 17 + k2];
-        for (int j = t; j < V * 16; j += kTileThreads) {
-          const int y = kX + (j >> 4);
-          float2 v[8];
+          for (int n2 = 0; n2 < 16; ++n2) gcv[n2] = r < Vr && ((xMask >> n2) & 1u) ? __ldg(src + 8 * n2) : 0.f;
+          if (wrapped && r < Vr && R0 + r >= 1) {
+            const float add = __ldg(sd->gWrap + o * (sd->dataH + 1) + R0 + r - 1);
 #pragma unroll
-          for (int k1 = 0; k1 < 8; ++k1) v[k1] = W[bwidx(y, 8 * k2 + k1)];
-          dft8<true>(v);
-#pragma unroll
-          for (int n1 = 0; n1 < 8; ++n1) W[bwidx(y, 8 * k2 + n1)] = n1 ? c_mulc(v[n1], twr[n1]) : v[0];
-        }
-      }
-      __syncthreads();
-      // I4 + the first pass of FFT(a): x-dim pass A' gives z = e + i o at the
-      // row's outputs x = n1 + 8 n2; a = dL/dC * z/|z| on the valid outputs
-      // (|z| as the forward computed it); then the forward x-dim pass A of a
-      // on the same 16 elements, in registers
-      for (int j = t; j < V * 8; j += kTileThreads) {
-        const int y = kX + (j >> 3), n1 = j & 7;
-        const int gy = R0 + y - kX;
-        // dL/dC of the item's valid outputs, loaded before the transform so
-        // that their latency overlaps it
-        float gcv[16];
-        {
-          const float* __restrict__ grow = sd->gC + (size_t)o * cStride + (size_t)gy * cPitch;
-#pragma unroll
-          for (int n2 = 0; n2 < 16; ++n2) {
-            const int x = n1 + 8 * n2, gx = C0 + x - kX;
-            gcv[n2] = (x >= kX && x < kX + V && gy < cRows && gx < cCols) ? __ldg(grow + gx) : 0.f;
-            if (wrapW && gx == 0 && gy >= 1 && gy < cRows) gcv[n2] += __ldg(sd->gWrap + o * (sd->dataH + 1) + gy - 1);
+            for (int n2 = 0; n2 < 16; ++n2)
+              if (n2 == (kX >> 3)) gcv[n2] += add;
           }
-        }
-        float2 v[16];
+          {
+            float2 twr[8];
 #pragma unroll
-        for (int k2 = 0; k2 < 16; ++k2) v[k2] = W[bwidx(y, 8 * k2 + n1)];
-        dft16<true>(v);
+            for (int m = 1; m < 8; ++m) twr[m] = tw[m * 17 + k2];
+#pragma unroll 1
+            for (int q = r0 + (lane >> 4); q < min(Vr, r0 + 4); q += 2) {
+              float2* wr = W + widx(kX + q, 8 * k2);
+              float2 v[8];
 #pragma unroll
-        for (int n2 = 0; n2 < 16; ++n2) {
-          const int x = n1 + 8 * n2;
-          const int gx = C0 + x - kX;
-          float2 a = make_float2(0.f, 0.f);
-          if (x >= kX && x < kX + V && gy < cRows && gx < cCols) {
-            const float gc = gcv[n2];
-            // |z| as the forward computes it (s * rsqrt(s)); 1/|z| is the
-            // same reciprocal square root, so a = gc z / |z| takes no division
-            const float sq = fmaf(v[n2].x, v[n2].x, v[n2].y * v[n2].y);
-            float rs;
-            asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(rs) : "f"(fmaxf(sq, 1e-30f)));
-            const float m = sq * rs;
-            if (m > kMagFloor) {
-              const float sc = gc * rs;
-              a = make_float2(sc * v[n2].x, sc * v[n2].y);
+              for (int k1 = 0; k1 < 8; ++k1) v[k1] = wr[k1];
+              dft8<true>(v);
+#pragma unroll
+              for (int m = 0; m < 8; ++m) wr[m] = m ? c_mulc(v[m], twr[m]) : v[0];
             }
           }
-          v[n2] = a;
+          __syncwarp();
+          if (r < Vr) {
+            float2* wr = W + widx(kX + r, n1);
+            float2 v[16];
+#pragma unroll
+            for (int m = 0; m < 16; ++m) v[m] = wr[9 * m];
+            dft16<true>(v);
+#pragma unroll
+            for (int n2 = 0; n2 < 16; ++n2) {
+              // |z| as the forward computes it (s * rsqrt(s)); 1/|z| is the
+              // same reciprocal square root, so a = gc z / |z| takes no
+              // division; outside the valid outputs gc is 0
+              const float sq = fmaf(v[n2].x, v[n2].x, v[n2].y * v[n2].y);
+              float rs;
+              asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(rs) : "f"(fmaxf(sq, 1e-30f)));
+              const float sc = gcv[n2] * rs;
+              v[n2] = ((xMask >> n2) & 1u) && sq * rs > kMagFloor ? make_float2(sc * v[n2].x, sc * v[n2].y)
+                                                                  : make_float2(0.f, 0.f);
+            }
+            dft16<false>(v);
+            // twiddles four at a time, read before the stores they scale
+#pragma unroll
+            for (int b = 0; b < 16; b += 4) {
+              float2 twr[4];
+#pragma unroll
+              for (int m = 0; m < 4; ++m) twr[m] = tw[n1 * 17 + b + m];
+#pragma unroll
+              for (int m = 0; m < 4; ++m) wr[9 * (b + m)] = c_mul(v[b + m], twr[m]);
+            }
+          }
+          __syncwarp();
+#pragma unroll 1
+          for (int q = r0 + (lane >> 4); q < min(Vr, r0 + 4); q += 2) {
+            float2* wq = W + widx(kX + q, 8 * k2);
+            float2 v[8];
+#pragma unroll
+            for (int m = 0; m < 8; ++m) v[m] = wq[m];
+            dft8<false>(v);
+#pragma unroll
+            for (int k1 = 0; k1 < 8; ++k1) wq[k1] = v[k1];
+          }
         }
-        dft16<false>(v);
-        float2 twr[16];
-#pragma unroll
-        for (int k2 = 0; k2 < 16; ++k2) twr[k2] = tw[n1 * 17 + k2];
-#pragma unroll
-        for (int k2 = 0; k2 < 16; ++k2) W[bwidx(y, n1 + 8 * k2)] = c_mul(v[k2], twr[k2]);
       }
       __syncthreads();
-      for (int j = t; j < V * 16; j += kTileThreads) {
-        const int y = kX + (j >> 4), k2 = j & 15;
-        float2 v[8];
-#pragma unroll
-        for (int n1 = 0; n1 < 8; ++n1) v[n1] = W[bwidx(y, 8 * k2 + n1)];
-        dft8<false>(v);
-#pragma unroll
-        for (int k1 = 0; k1 < 8; ++k1) W[bwidx(y, 8 * k2 + k1)] = v[k1];
-      }
-      __syncthreads();
+      // forward y-dim passes of a, each lane's column
 #pragma unroll
       for (int it = 0; it < 2; ++it) {
-        const int j = t + it * kTileThreads;
-        const int p = pcol, n1 = j >> 7;
+        const int n1 = h + 4 * it;
+        float2* col = W + widx(n1, pcol);
         float2 v[16];
 #pragma unroll
-        for (int m = 0; m < 16; ++m) v[m] = W[bwidx(n1 + 8 * m, p)];
+        for (int m = 0; m < 16; ++m) v[m] = col[8 * m * kWPitch];
         dft16<false>(v);
         float2 twr[16];
 #pragma unroll
         for (int k2 = 0; k2 < 16; ++k2) twr[k2] = tw[n1 * 17 + k2];
 #pragma unroll
-        for (int k2 = 0; k2 < 16; ++k2) W[bwidx(n1 + 8 * k2, p)] = c_mul(v[k2], twr[k2]);
+        for (int k2 = 0; k2 < 16; ++k2) col[8 * k2 * kWPitch] = c_mul(v[k2], twr[k2]);
       }
-      __syncthreads();
+      named_barrier(1 + quad, kTileThreads / 4);
+      // the first coefficients of the accumulation are under way during the last pass
+      const float4* __restrict__ cA = sd->bwA + (size_t)o * kSpecHalf;
+      const float2* __restrict__ cB = sd->bwB + (size_t)o * kSpecHalf;
+      const int sl = t & 63, pr = t >> 6;
+      auto fetch = [&](int r0, BwEntries& e) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int j = (pr + 8 * (r0 + u)) * kXhCols + sl;
+          e.c4[u] = __ldg(cA + j);
+          e.c2[u] = __ldg(cB + j);
+          e.X[u] = Xs[j];   // written by this CTA for this item: a coherent load
+        }
+      };
+      BwEntries next;
+      fetch(0, next);
 #pragma unroll
       for (int it = 0; it < 4; ++it) {
-        const int j = t + it * kTileThreads;
-        const int p = pcol, k2 = j >> 7;
+        float2* col = W + widx(8 * (h + 4 * it), pcol);
         float2 v[8];
 #pragma unroll
-        for (int n1 = 0; n1 < 8; ++n1) v[n1] = W[bwidx(8 * k2 + n1, p)];
+        for (int n1 = 0; n1 < 8; ++n1) v[n1] = col[n1 * kWPitch];
         dft8<false>(v);
 #pragma unroll
-        for (int k1 = 0; k1 < 8; ++k1) W[bwidx(8 * k2 + k1, p)] = v[k1];
+        for (int k1 = 0; k1 < 8; ++k1) col[k1 * kWPitch] = v[k1];
       }
       __syncthreads();
       // Hermitian accumulation and the parameter dot products.  Entry j of
       // the half layout holds k = (ky, kx), kx in [0, 64]; its partner -k
       // covers the columns 65..127, so every frequency enters the dot
       // products once (columns 0 and 64 pair with themselves: their -k
-      // coefficients are 0).  X is Hermitian, X(-k) = conj(X(k)).
+      // coefficients are 0).  X is Hermitian, X(-k) = conj(X(k)).  Thread t
+      // owns slot t mod 64 and the rows py = t / 64 + 8 r; four entries at a
+      // time, the next four's loads issued before them.
       {
-        const float4* __restrict__ cA = sd->bwA + (size_t)o * kSpecHalf;
-        const float2* __restrict__ cB = sd->bwB + (size_t)o * kSpecHalf;
         float sa = 0.f, sr = 0.f;
-        // entry (py, sl) of the half layout, j = py * kXhCols + sl
-        auto entry = [&](int py, int sl, int p, int np, int wp) {
-          const int j = py * kXhCols + sl;
-          const float4 c4 = __ldg(cA + j);   // G(k), G(-k), dGa(k), dGr(k)
-          const float2 c2 = __ldg(cB + j);   // dGa(-k), dGr(-k)
-          const float2 X = Xs[j];   // written by this CTA for this tile: a coherent load
-          const int ky = 16 * (py & 7) + (py >> 3);
-          const int npy = perm128d((kTile - ky) & 127);
-          const float2 A1 = W[wp], A2 = W[bwidx(npy, np)];
-          const float2 bb = Bh[j];
-          Bh[j] = make_float2(fmaf(0.5f * c4.x, A1.x, fmaf(0.5f * c4.y, A2.x, bb.x)),
-                              fmaf(0.5f * c4.x, A1.y, fmaf(-0.5f * c4.y, A2.y, bb.y)));
-          const float re1 = A1.x * X.x + A1.y * X.y;   // Re(conj(A(k)) X(k))
-          const float re2 = A2.x * X.x - A2.y * X.y;   // Re(conj(A(-k)) conj(X(k)))
-          sa = fmaf(c4.z, re1, fmaf(c2.x, re2, sa));
-          sr = fmaf(c4.w, re1, fmaf(c2.y, re2, sr));
-        };
-        // slots 0..63: thread t owns slot sl = t mod 64 and the rows
-        // py = t / 64 + 8 r (r = 0..15), so its column terms are fixed
-        // Four entries at a time: all their loads first, then the updates
-        // (the entries' Bh words are distinct, but a store would otherwise
-        // hold back the next entry's shared-memory loads).
-        {
-          const int sl = t & 63, pr = t >> 6;
-          const int kx = half_group(sl) + 16 * (sl & 3);
-          const int p = perm128d(kx), np = perm128d((kTile - kx) & 127);
-          const int pp = bwidx(pr & 1, p) - (pr & 1) * kTile;
-#pragma unroll 1
-          for (int r0 = 0; r0 < 16; r0 += 4) {
-            float4 c4[4];
-            float2 c2[4], X[4], A1[4], A2[4], bb[4];
+        const int kx = half_group(sl) + 16 * (sl & 3);
+        const float2* W1 = W + widx(pr, perm128d(kx));
+        const float2* W2 = W + widx(0, perm128d((kTile - kx) & 127));
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              const int py = pr + 8 * (r0 + u);
-              const int j = py * kXhCols + sl;
-              c4[u] = __ldg(cA + j);
-              c2[u] = __ldg(cB + j);
-              X[u] = Xs[j];
-              const int ky = 16 * (py & 7) + (py >> 3);
-              A1[u] = W[py * kTile + pp];
-              A2[u] = W[bwidx(perm128d((kTile - ky) & 127), np)];
-              bb[u] = Bh[j];
-            }
+        for (int r0 = 0; r0 < 16; r0 += 4) {
+          BwEntries e = next;
+          if (r0 + 4 < 16) fetch(r0 + 4, next);
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              const int j = (pr + 8 * (r0 + u)) * kXhCols + sl;
-              Bh[j] = make_float2(fmaf(0.5f * c4[u].x, A1[u].x, fmaf(0.5f * c4[u].y, A2[u].x, bb[u].x)),
-                                  fmaf(0.5f * c4[u].x, A1[u].y, fmaf(-0.5f * c4[u].y, A2[u].y, bb[u].y)));
-              const float re1 = A1[u].x * X[u].x + A1[u].y * X[u].y;
-              const float re2 = A2[u].x * X[u].x - A2[u].y * X[u].y;
-              sa = fmaf(c4[u].z, re1, fmaf(c2[u].x, re2, sa));
-              sr = fmaf(c4[u].w, re1, fmaf(c2[u].y, re2, sr));
-            }
+          for (int u = 0; u < 4; ++u) {
+            const int py = pr + 8 * (r0 + u), j = py * kXhCols + sl;
+            const int ky = 16 * (py & 7) + (py >> 3);
+            const float2 A1 = W1[8 * (r0 + u) * kWPitch], A2 = W2[perm128d((kTile - ky) & 127) * kWPitch];
+            const float2 bb = Bh[j];
+            Bh[j] = make_float2(fmaf(0.5f * e.c4[u].x, A1.x, fmaf(0.5f * e.c4[u].y, A2.x, bb.x)),
+                                fmaf(0.5f * e.c4[u].x, A1.y, fmaf(-0.5f * e.c4[u].y, A2.y, bb.y)));
+            const float re1 = A1.x * e.X[u].x + A1.y * e.X[u].y;   // Re(conj(A(k)) X(k))
+            const float re2 = A2.x * e.X[u].x - A2.y * e.X[u].y;   // Re(conj(A(-k)) conj(X(k)))
+            sa = fmaf(e.c4[u].z, re1, fmaf(e.c2[u].x, re2, sa));
+            sr = fmaf(e.c4[u].w, re1, fmaf(e.c2[u].y, re2, sr));
           }
         }
-        // the Nyquist slot 64 (kx = 64): one row per thread of the first 128
+        // slot 64 (kx = 64): one row for each of the first 128 threads
         if (t < kTile) {
-          const int p = perm128d(64), sl = t & 63;
-          const int row = (t & 64) + 4 * half_group(sl) + (sl & 3);
-          entry(row, 64, p, p, bwidx(row, p));
+          const int py = (t & 64) + 4 * half_group(sl) + (sl & 3), j = py * kXhCols + 64;
+          const int ky = 16 * (py & 7) + (py >> 3), p = perm128d(64);
+          const float4 c4 = __ldg(cA + j);
+          const float2 c2 = __ldg(cB + j), X = Xs[j];
+          const float2 A1 = W[widx(py, p)], A2 = W[widx(perm128d((kTile - ky) & 127), p)], bb = Bh[j];
+          Bh[j] = make_float2(fmaf(0.5f * c4.x, A1.x, fmaf(0.5f * c4.y, A2.x, bb.x)),
+                              fmaf(0.5f * c4.x, A1.y, fmaf(-0.5f * c4.y, A2.y, bb.y)));
+          const float re1 = A1.x * X.x + A1.y * X.y, re2 = A2.x * X.x - A2.y * X.y;
+          sa = fmaf(c4.z, re1, fmaf(c2.x, re2, sa));
+          sr = fmaf(c4.w, re1, fmaf(c2.y, re2, sr));
         }
         accA += sa;
         accR += sr;
       }
-      // no barrier: every Bh entry has one owner thread, and the next
-      // orientation's I1 touches only TMEM until its barrier
+      // this warp no longer reads W (the item's last orientation is ordered by
+      // the barrier below)
+      __syncwarp();
+      if (lane == 0 && o + 1 < oE) mbar_arrive(barW);
     }
     __syncthreads();
     // one inverse transform of the Hermitian sum: Re -> window gradient,
     // scattered to the float level through the padded-torus index maps.
     // This lane's column of the full spectrum is read from the half Bh
-    // without a branch (conj(Bh(-k)) for kx > 64).
-    const HalfColumn hc(pcol);
-    const bool pConj = hc.conj;
-    const int pSlot = hc.slot;
-    const float pSign = pConj ? -1.f : 1.f;
+    // without a branch (conj(Bh(-k)) for mirrored columns).
+    {
+      const HalfColumn hc(pcol);
+      const float sign = hc.conj ? -1.f : 1.f;
+#pragma unroll 1
+      for (int it = 0; it < 4; ++it) {
+        const int k2 = h + 4 * it;
+        float2 v[8];
 #pragma unroll
-    for (int it = 0; it < 4; ++it) {
-      const int j = t + it * kTileThreads;
-      const int p = pcol, k2 = j >> 7;
-      float2 v[8];
+        for (int k1 = 0; k1 < 8; ++k1) {
+          const int row = hc.conj ? (k2 > 0 ? 8 * (16 - k2) + (7 - k1) : (8 - k1) & 7) : 8 * k2 + k1;
+          v[k1] = Bh[row * kXhCols + hc.slot];
+          v[k1].y *= sign;
+        }
+        dft8<true>(v);
 #pragma unroll
-      for (int k1 = 0; k1 < 8; ++k1) {
-        const int row = pConj ? (k2 > 0 ? 8 * (16 - k2) + (7 - k1) : (8 - k1) & 7) : 8 * k2 + k1;
-        v[k1] = Bh[row * kXhCols + pSlot];
-        v[k1].y *= pSign;
+        for (int n1 = 0; n1 < 8; ++n1) W[widx(8 * k2 + n1, pcol)] = c_mulc(v[n1], tw[n1 * 17 + k2]);
       }
-      dft8<true>(v);
-#pragma unroll
-      for (int n1 = 0; n1 < 8; ++n1) W[bwidx(8 * k2 + n1, p)] = c_mulc(v[n1], tw[n1 * 17 + k2]);
     }
-    __syncthreads();
+    named_barrier(1 + quad, kTileThreads / 4);
 #pragma unroll
     for (int it = 0; it < 2; ++it) {
-      const int j = t + it * kTileThreads;
-      const int p = pcol, n1 = j >> 7;
+      const int n1 = h + 4 * it;
+      float2* col = W + widx(n1, pcol);
       float2 v[16];
 #pragma unroll
-      for (int k2 = 0; k2 < 16; ++k2) v[k2] = W[bwidx(8 * k2 + n1, p)];
+      for (int k2 = 0; k2 < 16; ++k2) v[k2] = W[widx(8 * k2 + n1, pcol)];
       dft16<true>(v);
 #pragma unroll
-      for (int n2 = 0; n2 < 16; ++n2) W[bwidx(n1 + 8 * n2, p)] = v[n2];
+      for (int n2 = 0; n2 < 16; ++n2) col[8 * n2 * kWPitch] = v[n2];
     }
     __syncthreads();
+    // x-passes: eight rows to a warp
+    {
+      float* __restrict__ gl = sd->gLvl;
+      const int gp = sd->lvlPitchF, k2 = lane & 15, n1 = lane & 7;
+#pragma unroll 1
+      for (int r0 = 8 * warp; r0 < 8 * warp + 8; r0 += 4) {
+#pragma unroll 1
+        for (int y = r0 + (lane >> 4); y < r0 + 4; y += 2) {
+          float2* wr = W + widx(y, 8 * k2);
+          float2 v[8];
 #pragma unroll
-    for (int it = 0; it < 4; ++it) {
-      const int j = t + it * kTileThreads;
-      const int y = j >> 4, k2 = j & 15;
-      float2 v[8];
+          for (int k1 = 0; k1 < 8; ++k1) v[k1] = wr[k1];
+          dft8<true>(v);
 #pragma unroll
-      for (int k1 = 0; k1 < 8; ++k1) v[k1] = W[bwidx(y, 8 * k2 + k1)];
-      dft8<true>(v);
+          for (int m = 0; m < 8; ++m) wr[m] = c_mulc(v[m], tw[m * 17 + k2]);
+        }
+        __syncwarp();
+        const int y = r0 + (lane >> 3);
+        const float2* wr = W + widx(y, n1);
+        float2 v[16];
 #pragma unroll
-      for (int n1 = 0; n1 < 8; ++n1) W[bwidx(y, 8 * k2 + n1)] = c_mulc(v[n1], tw[n1 * 17 + k2]);
-    }
-    __syncthreads();
-    float* __restrict__ gl = sd->gLvl;
-    const int gp = sd->lvlPitchF;
+        for (int m = 0; m < 16; ++m) v[m] = wr[9 * m];
+        dft16<true>(v);
+        float* row = gl + (size_t)rmap[y] * gp;
 #pragma unroll
-    for (int it = 0; it < 2; ++it) {
-      const int j = t + it * kTileThreads;
-      const int y = j >> 3, n1 = j & 7;
-      float2 v[16];
-#pragma unroll
-      for (int k2 = 0; k2 < 16; ++k2) v[k2] = W[bwidx(y, 8 * k2 + n1)];
-      dft16<true>(v);
-      float* row = gl + (size_t)rmap[y] * gp;
-#pragma unroll
-      for (int n2 = 0; n2 < 16; ++n2) {
-        const float g = v[n2].x;
-        if (g != 0.f) atomicAdd(row + cmap[n1 + 8 * n2], kFloatLevelScale * g);
+        for (int n2 = 0; n2 < 16; ++n2) {
+          const float g = v[n2].x;
+          if (g != 0.f) atomicAdd(row + cmap[n1 + 8 * n2], kFloatLevelScale * g);
+        }
       }
     }
   }

@@ -138,7 +138,8 @@ bool build_scales(int width, int height, const std::vector<float>& lambdas_in,
 // the tensor-memory lanes that hold them, rows in groups of four.
 void tile_spectrum(const std::vector<float>* even, const std::vector<float>* odd, int kW, int kX,
                    std::vector<float>& out) {
-  const int T = kTile, n = kW, h = kX;
+  constexpr int T = kTile;
+  const int n = kW, h = kX;
   std::vector<double> cs(T), sn(T);
   for (int m = 0; m < T; ++m) {
     cs[m] = std::cos(2.0 * M_PI * m / T);
@@ -162,16 +163,19 @@ void tile_spectrum(const std::vector<float>* even, const std::vector<float>* odd
         rim[row * T + kx] = im;
       }
     }
+    // columns side by side (each one's sum over the rows in the same order)
+    float* spec = out.data() + static_cast<size_t>(o) * T * T;
+    double re[T];
     for (int ky = 0; ky < T; ++ky) {
-      for (int kx = 0; kx < T; ++kx) {
-        double re = 0;
-        for (int row = 0; row < n; ++row) {
-          const int m = ((ky * (row - h)) % T + T) % T;
-          re += rre[row * T + kx] * cs[m] + rim[row * T + kx] * sn[m];
-        }
-        out[static_cast<size_t>(o) * T * T + spectrum_pos(perm128(ky), perm128(kx))] =
-            static_cast<float>(re / (double(T) * T));
+      std::fill(re, re + T, 0.0);
+      for (int row = 0; row < n; ++row) {
+        const int m = ((ky * (row - h)) % T + T) % T;
+        const double c = cs[m], s = sn[m];
+        const double *pr = &rre[row * T], *pi = &rim[row * T];
+        for (int kx = 0; kx < T; ++kx) re[kx] += pr[kx] * c + pi[kx] * s;
       }
+      const int py = perm128(ky);
+      for (int kx = 0; kx < T; ++kx) spec[spectrum_pos(py, perm128(kx))] = static_cast<float>(re[kx] / (double(T) * T));
     }
   }
 }

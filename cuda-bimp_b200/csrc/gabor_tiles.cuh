@@ -274,35 +274,50 @@ __device__ __forceinline__ int window_src(int o, int i, int fft, int nData, int 
   return pad_src(pmod(o + i, fft), nData, kHalf);
 }
 
-// The columns [iA, iB) of a window that lie inside the data.
+// The columns [iA, iB) of a window that are staged as 16-byte chunks: those
+// whose chunk lies inside the data, or all of them.
+template <bool FLT>
 struct WindowSpan {
-  int iA, iB;
+  static constexpr int kVals = 16 / sizeof(typename RawWindow<FLT>::T);   // values of a chunk
+  int c0, iA, iB, end;   // end: chunks past it are not read
   __device__ __forceinline__ WindowSpan(const ScaleDev* sd, int C0) {
-    iA = min(max(sd->kX - C0, 0), kTile);
-    iB = max(iA, min(sd->dataW - (C0 - sd->kX), kTile));
+    c0 = C0 - sd->kX;
+    const bool endInside = c0 + kTile <= sd->dataW;
+    end = endInside ? c0 + kTile : sd->dataW & ~(kVals - 1);
+    iA = min(max(-c0, 0), kTile);
+    iB = endInside ? kTile : max(iA, end - c0);
   }
   __device__ __forceinline__ bool all() const { return iA == 0 && iB == kTile; }
 };
-// A byte window's data columns are staged as aligned 16-byte chunks (level
-// rows start 16-byte aligned and their pitch is a multiple of 16), asynchronously,
-// so that the window of the CTA's next item lands during the item before it:
-// column i of row r goes to raw[r * kPitch + lead + i], lead = (C0 - kX) mod
-// 16.  Chunks that reach past the data stay inside their row.
-__device__ __forceinline__ void raw_chunks_load(const ScaleDev* sd, int R0, int C0, uint8_t* raw, int t) {
-  const int kX = sd->kX, r0 = R0 - kX, c0 = C0 - kX, pitch = sd->lvlPitch;
-  // four threads a row: chunks l, l + 4, and (l = 0) the 9th
-  const int r = t >> 2, l = t & 3;
+// A window's data columns are staged as aligned 16-byte chunks (level rows
+// start 16-byte aligned and their pitch is a multiple of 16 bytes),
+// asynchronously: column i of row r goes to raw[r * kPitch + lead + i], lead =
+// C0 - kX modulo the values of a chunk.  (A window that ends inside the data
+// may read its last chunk past the data, inside the row's pitch.)
+template <bool FLT>
+__device__ __forceinline__ void raw_chunks_load(const ScaleDev* sd, int R0, int C0, typename RawWindow<FLT>::T* raw,
+                                                int t) {
+  using T = typename RawWindow<FLT>::T;
+  constexpr int kVals = WindowSpan<FLT>::kVals, kChunks = kTile / kVals + 1;
+  const WindowSpan<FLT> span(sd, C0);
+  const int kX = sd->kX, r0 = R0 - kX;
+  const T* lvl;
+  int pitch;
+  if constexpr (FLT) { lvl = sd->lvlF; pitch = sd->lvlPitchF; }
+  else { lvl = sd->lvl; pitch = sd->lvlPitch; }
+  // four threads a row
+  const int r = t >> 2;
   const int row = r0 >= 0 && r0 + kTile <= sd->dataH ? r0 + r : window_src(r0, r, sd->fftH, sd->dataH, kX);
-  const uint8_t* src = sd->lvl + (size_t)row * pitch;
-  raw += r * RawWindow<false>::kPitch;
+  const T* src = lvl + (size_t)row * pitch;
+  raw += r * RawWindow<FLT>::kPitch;
 #pragma unroll
-  for (int c = l; c < 9; c += 4) {
-    const int x = (c0 & ~15) + 16 * c;
-    if (x >= 0 && x < pitch && x < c0 + kTile) cp_async16(raw + 16 * c, src + x);
+  for (int c = t & 3; c < kChunks; c += 4) {
+    const int x = (span.c0 & ~(kVals - 1)) + kVals * c;
+    if (x >= 0 && x < span.end) cp_async16(raw + kVals * c, src + x);
   }
 }
-// The window's columns outside [iA, iB), value by value through the
-// padded-torus map: warp w stages rows w, w + 16, ..., lane l the columns l,
+// The window's columns outside [iA, iB) (which no chunk writes), value by value
+// through the padded-torus map: warp w stages rows w, w + 16, ..., lane l the columns l,
 // l + 32, l + 64, l + 96 among them.
 template <bool FLT>
 __device__ __forceinline__ void raw_window_copy(const ScaleDev* sd, int R0, int C0, typename RawWindow<FLT>::T* raw,
@@ -517,7 +532,7 @@ k_gabor_tiles(const ScaleDev* __restrict__ sds, const TileWork* __restrict__ wor
 
   if constexpr (!FLT) {
     const int tile = qItem[0].tile, ty = tile / qScale->tilesX, tx = tile - ty * qScale->tilesX;
-    raw_chunks_load(qScale, ty * qScale->V, tx * qScale->V, rawG, t);
+    raw_chunks_load<false>(qScale, ty * qScale->V, tx * qScale->V, rawG, t);
   }
 
   for (int w = blockIdx.x, slot = 0; w < nwork; w += gridDim.x, slot ^= 1) {
@@ -552,12 +567,16 @@ k_gabor_tiles(const ScaleDev* __restrict__ sds, const TileWork* __restrict__ wor
     if constexpr (FLT) {
       load_first();
       float* raw = reinterpret_cast<float*>(W + PadLayout::kHalf);
-      raw_window_copy<FLT>(sd, R0, C0, raw, 0, 0, t);
+      raw_chunks_load<FLT>(sd, R0, C0, raw, t);
+      raw += (C0 - kX) & 3;
+      const WindowSpan<FLT> span(sd, C0);
+      if (!span.all()) raw_window_copy<FLT>(sd, R0, C0, raw, span.iA, span.iB, t);
+      cp_async_wait();
       __syncthreads();
       tile_forward_spectrum<FLT, false, PadLayout>(raw, W, Nyq, tw, tlane, nullptr, t, [] {});
     } else {
       uint8_t* raw = rawG + ((C0 - kX) & 15);
-      const WindowSpan span(sd, C0);
+      const WindowSpan<FLT> span(sd, C0);
       if (!span.all()) {
         raw_window_copy<FLT>(sd, R0, C0, raw, span.iA, span.iB, t);
         __syncthreads();
@@ -668,7 +687,7 @@ k_gabor_tiles(const ScaleDev* __restrict__ sds, const TileWork* __restrict__ wor
         const ScaleDev* nsd = qScale + (slot ^ 1);
         if (nx.oBegin < nx.oEnd) {
           const int ny = nx.tile / nsd->tilesX, nX = nx.tile - ny * nsd->tilesX;
-          raw_chunks_load(nsd, ny * nsd->V, nX * nsd->V, rawG, t);
+          raw_chunks_load<false>(nsd, ny * nsd->V, nX * nsd->V, rawG, t);
         }
       }
       // The x-passes, four valid rows to a warp at a time: I3 (pass B', two
