@@ -20,6 +20,7 @@
 #include "bimp_b200_adjoint.h"
 #include "bimp_internal.h"
 #include "kernels.h"
+#include "tile_plan.h"
 
 using namespace bimp_b200;
 
@@ -71,6 +72,15 @@ struct bimp_adjoint {
   size_t bytes = 0;
   std::vector<ScaleDev> h_sd;
   ScaleDev* d_sd = nullptr;
+  // The tile kernels' work plans, one per chunk of images: the balanced split
+  // over one persistent CTA per SM (with one CTA or one whole tile at a time,
+  // the 451 tiles of a 1333 x 1001 image took four waves for 3.05 and two
+  // small images a whole tile's eight orientations in a row)
+  struct Plan {
+    size_t first = 0;   // in d_tiles
+    int items = 0, grid = 0;
+  };
+  std::vector<Plan> fwdPlan, bwdPlan;
   TileWork* d_tiles = nullptr;
   int nTiles = 0;
   int2* d_sten = nullptr;                 // forward stencil blocks (data)
@@ -240,13 +250,27 @@ struct bimp_adjoint {
     nTiles = static_cast<int>(tiles.size());
     nSten = static_cast<int>(sten.size());
     nStenB = static_cast<int>(stenB.size());
+    std::vector<TileWork> plans;
+    for (int i0 = 0; i0 < n; i0 += chunk) {
+      const std::vector<TileWork> part(tiles.begin() + tileStart[i0], tiles.begin() + tileStart[std::min(n, i0 + chunk)]);
+      auto add = [&](std::vector<Plan>& to, const TileCost& cost) {
+        Plan p;
+        const std::vector<TileWork> work = split_plan(part, sds, cost, num_sms(), &p.grid);
+        p.first = plans.size();
+        p.items = static_cast<int>(work.size());
+        plans.insert(plans.end(), work.begin(), work.end());
+        to.push_back(p);
+        return p.grid;
+      };
+      add(fwdPlan, kForwardCost);
+      bwdGrid = std::max(bwdGrid, add(bwdPlan, kBackwardCost));
+    }
     const size_t offSd = take(sizeof(ScaleDev) * sds.size());
-    const size_t offT2 = take(sizeof(TileWork) * tiles.size());
+    const size_t offT2 = take(sizeof(TileWork) * plans.size());
     const size_t offSt = take(sizeof(int2) * sten.size());
     const size_t offStB = take(sizeof(int2) * stenB.size());
     const size_t offPyr = take(sizeof(PyrJobF) * std::max(1, maxLevel * n));
     const size_t offPyrA = take(sizeof(PyrJobF) * std::max(1, maxLevel * n));
-    bwdGrid = std::max(1, std::min(nTiles, num_sms()));
     const size_t offXs = take(sizeof(float2) * (size_t)bwdGrid * kSpecHalf);
     const size_t offLoss = take(sizeof(double) * 8);
     const size_t offMax = take(sizeof(unsigned int) * (sds.size() + 1));
@@ -321,7 +345,7 @@ struct bimp_adjoint {
     ADJ_CUDA(cudaMemcpy(dBB, hB.data(), sizeof(float2) * hB.size(), cudaMemcpyHostToDevice));
     ADJ_CUDA(cudaMemcpy(d_sd, sds.data(), sizeof(ScaleDev) * sds.size(), cudaMemcpyHostToDevice));
     ADJ_CUDA(cudaMemcpy(b + offMaps, maps.data(), kTensorMapBytes * sds.size(), cudaMemcpyHostToDevice));
-    ADJ_CUDA(cudaMemcpy(d_tiles, tiles.data(), sizeof(TileWork) * tiles.size(), cudaMemcpyHostToDevice));
+    ADJ_CUDA(cudaMemcpy(d_tiles, plans.data(), sizeof(TileWork) * plans.size(), cudaMemcpyHostToDevice));
     ADJ_CUDA(cudaMemcpy(d_sten, sten.data(), sizeof(int2) * sten.size(), cudaMemcpyHostToDevice));
     ADJ_CUDA(cudaMemcpy(d_stenB, stenB.data(), sizeof(int2) * stenB.size(), cudaMemcpyHostToDevice));
     std::vector<PyrJobF> fj, aj;
@@ -358,7 +382,8 @@ struct bimp_adjoint {
     unsigned int* fault = d_max + h_sd.size();
     for (int i0 = 0; i0 < n; i0 += chunk) {
       const int i1 = std::min(n, i0 + chunk);
-      launch_gabor_flt(d_sd, d_tiles + tileStart[i0], tileStart[i1] - tileStart[i0], fault, s, pipelined);
+      const Plan& p = fwdPlan[i0 / chunk];
+      launch_gabor_flt(d_sd, d_tiles + p.first, p.items, p.grid, fault, s, pipelined);
       launch_stencil(d_sd, d_sten + stenStart[i0], stenStart[i1] - stenStart[i0], fault, s, kStencilAdj);
       launch_masked_loss(d_sd, d_sten + stenStart[i0], stenStart[i1] - stenStart[i0], d_loss, d_gp, s);
     }
@@ -375,7 +400,8 @@ struct bimp_adjoint {
     for (int i0 = 0; i0 < n; i0 += chunk) {
       const int i1 = std::min(n, i0 + chunk);
       launch_stencil_bwd(d_sd, d_stenB + stenBStart[i0], stenBStart[i1] - stenBStart[i0], s);
-      launch_gabor_bwd(d_sd, d_tiles + tileStart[i0], tileStart[i1] - tileStart[i0], bwdGrid, d_xscr, d_gp, s);
+      const Plan& p = bwdPlan[i0 / chunk];
+      launch_gabor_bwd(d_sd, d_tiles + p.first, p.items, p.grid, d_xscr, d_gp, s);
     }
     for (int l = maxLevel; l >= 1; --l) launch_pyr_f_adj(d_pyrAdj + (l - 1) * n, n, lw[l], lh[l], s);
     ADJ_CUDA(cudaMemcpy2DAsync(grad, sizeof(float) * pitch, d_glvl, sizeof(float) * lp[0], sizeof(float) * W,

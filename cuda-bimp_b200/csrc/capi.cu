@@ -16,6 +16,7 @@
 #include "bimp_b200_batch.h"
 #include "bimp_internal.h"
 #include "kernels.h"
+#include "tile_plan.h"
 
 using namespace bimp_b200;
 
@@ -161,72 +162,6 @@ struct Engine {
     const int v32 = vmax / 32 * 32;
     return (policy == 1 && v32 * 4 >= vmax * 3) ? v32 : vmax;
   }
-  // Balanced plan for a persistent grid of `grid` CTAs.  The (tile,
-  // orientation) pairs, tile by tile in plan order, are cut into at most
-  // `grid` contiguous runs of about equal cost; a run becomes one work item
-  // per tile it touches (a tile cut between two CTAs is transformed forward by
-  // both).  Costs are a fit to the kernel's measured item times (1080p, cycles;
-  // residual 1.7 k of about 90 k an item): 14.5 k for an item's forward
-  // transform, and per orientation 5.0 k + 0.77 k for each block of four rows
-  // (of the rows inside the map) on the scheduler with most of them; in units
-  // of an orientation of a V = 100 tile.  The weights before the x-passes went
-  // warp by warp left 3840 x 2160 at 946 us, these 859.  The smallest run bound
-  // that fits in `grid` runs is found by bisection.  Item k of CTA b is
-  // placed at index k * grid + b (the kernel strides its work list by the
-  // grid); CTAs with fewer items get empty ones.  *usedGrid receives the
-  // number of CTAs with work.
-  static std::vector<TileWork> split_plan(const std::vector<TileWork>& tiles, const std::vector<ScaleDev>& sds,
-                                          int grid, int* usedGrid) {
-    const double kFwd = 1.4;
-    std::vector<double> ori(tiles.size());
-    double total = 0.0, worst = 0.0;
-    for (size_t i = 0; i < tiles.size(); ++i) {
-      const ScaleDev& d = sds[tiles[i].entry];
-      const int ty = tiles[i].tile / d.tilesX;
-      const int vr = std::min(d.V, d.cRows - ty * d.V);   // valid rows inside the map (the x-passes' rows)
-      const int blocks = ((vr + 3) / 4 + 3) / 4;   // four-row blocks of the busiest scheduler
-      ori[i] = 0.481 + 0.0741 * blocks;
-      total += kNumOri * ori[i] + kFwd;
-      worst = std::max(worst, ori[i] + kFwd);
-    }
-    // greedy runs of the pair sequence under bound tau (a pair joins the
-    // current run while the run stays within tau); returns the run count
-    auto cut = [&](double tau, std::vector<std::vector<TileWork>>* runs) {
-      int n = 0;
-      double acc = 0.0;
-      for (size_t i = 0; i < tiles.size(); ++i)
-        for (int o = 0; o < kNumOri;) {
-          if (n == 0 || (acc + kFwd + ori[i] > tau && acc > 0.0)) {
-            ++n;
-            acc = 0.0;
-            if (runs) runs->emplace_back();
-          }
-          acc += kFwd + ori[i];   // the item's forward transform and first orientation
-          int k = 1 + static_cast<int>(std::floor(std::max(0.0, tau - acc) / ori[i]));
-          k = std::min(k, kNumOri - o);
-          acc += (k - 1) * ori[i];
-          if (runs) runs->back().push_back({tiles[i].entry, tiles[i].tile, o, o + k});
-          o += k;
-        }
-      return n;
-    };
-    double lo = std::max(worst, total / std::max(1, grid)) * 0.999, hi = total + worst;
-    for (int it = 0; it < 60 && hi - lo > 1e-6 * hi; ++it) {
-      const double mid = 0.5 * (lo + hi);
-      if (cut(mid, nullptr) <= grid) hi = mid;
-      else lo = mid;
-    }
-    std::vector<std::vector<TileWork>> runs;
-    cut(hi, &runs);
-    const int g = static_cast<int>(runs.size());
-    size_t depth = 0;
-    for (auto& r : runs) depth = std::max(depth, r.size());
-    std::vector<TileWork> out(depth * (size_t)g, TileWork{0, 0, 0, 0});
-    for (int b = 0; b < g; ++b)
-      for (size_t k = 0; k < runs[b].size(); ++k) out[k * (size_t)g + b] = runs[b][k];
-    *usedGrid = g;
-    return out;
-  }
   static std::vector<TileWork> tile_plan(std::vector<ScaleDev>& sds, int policy, int order) {
     std::vector<std::vector<TileWork>> per(sds.size());
     for (size_t e = 0; e < sds.size(); ++e) {
@@ -256,7 +191,7 @@ struct Engine {
     std::vector<TileWork> tiles = tile_plan(sds, policy, order);
     *nTilesOut = static_cast<int>(tiles.size());
     *gridOut = static_cast<int>(tiles.size());
-    if (grid > 0 && !tiles.empty()) return split_plan(tiles, sds, grid, gridOut);
+    if (grid > 0 && !tiles.empty()) return split_plan(tiles, sds, kForwardCost, grid, gridOut);
     return tiles;
   }
   int retile(int policy, int order, int grid, int kernel = 0) {
@@ -464,7 +399,7 @@ struct Engine {
     if (const char* g = std::getenv("BIMP_TILE_GRID")) defGrid = std::atoi(g);
     std::vector<TileWork> work = tiles;
     tileGrid = nTiles;
-    if (defGrid > 0 && !tiles.empty()) work = split_plan(tiles, sds, defGrid, &tileGrid);
+    if (defGrid > 0 && !tiles.empty()) work = split_plan(tiles, sds, kForwardCost, defGrid, &tileGrid);
     nWork = static_cast<int>(work.size());
     tileGridReq = std::max(0, defGrid);
     nSten = static_cast<int>(sten.size());

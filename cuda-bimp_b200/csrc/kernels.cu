@@ -1321,13 +1321,13 @@ void launch_gabor(const ScaleDev* d_sd, const TileWork* d_work, int nwork, int g
     launch_ex(k_gabor_tiles<false, false>, grid, kTileThreads, gabor_smem_bytes(), s, pdl, d_sd, d_work, nwork,
               d_fault);
 }
-void launch_gabor_flt(const ScaleDev* d_sd, const TileWork* d_work, int nwork, unsigned int* d_fault,
+void launch_gabor_flt(const ScaleDev* d_sd, const TileWork* d_work, int nwork, int grid, unsigned int* d_fault,
                       cudaStream_t s, bool pipelined) {
   if (nwork <= 0) return;
   if (pipelined)
-    k_gabor_tiles_ws<true><<<nwork, kTileThreads, kWsSmem, s>>>(d_sd, d_work, nwork);
+    k_gabor_tiles_ws<true><<<grid, kTileThreads, kWsSmem, s>>>(d_sd, d_work, nwork);
   else
-    k_gabor_tiles<true, false><<<nwork, kTileThreads, gabor_smem_bytes(), s>>>(d_sd, d_work, nwork, d_fault);
+    k_gabor_tiles<true, false><<<grid, kTileThreads, gabor_smem_bytes(), s>>>(d_sd, d_work, nwork, d_fault);
 }
 void launch_gabor_keep_z(const ScaleDev* d_sd, const TileWork* d_work, int nwork, unsigned int* d_fault,
                          cudaStream_t s) {
@@ -1358,7 +1358,7 @@ void launch_stencil_bwd(const ScaleDev* d_sd, const int2* d_work, int nwork, cud
 void launch_gabor_bwd(const ScaleDev* d_sd, const TileWork* d_work, int nwork, int grid, float2* d_xscratch,
                       double* d_gparams, cudaStream_t s) {
   if (nwork > 0)
-    k_gabor_tiles_bwd<<<std::min(grid, nwork), kTileThreads, kGaborBwdSmem, s>>>(d_sd, d_work, nwork, d_xscratch,
+    k_gabor_tiles_bwd<<<grid, kTileThreads, kGaborBwdSmem, s>>>(d_sd, d_work, nwork, d_xscratch,
                                                                                  d_gparams);
 }
 void launch_stencil(const ScaleDev* d_sd, const int2* d_work, int nwork, unsigned int* d_fault, cudaStream_t s,

@@ -97,9 +97,9 @@ void launch_nms(const ScaleDev* d_sd, const int2* d_rows, int nrows, int* d_coun
 // differentiable path and its adjoint
 void launch_pyr_f(const PyrJobF* d_jobs, int njobs, int maxW, int maxH, cudaStream_t s);
 void launch_pyr_f_adj(const PyrJobF* d_jobs, int njobs, int maxW, int maxH, cudaStream_t s);
-// differentiable forward: the tile kernel on the float levels (one CTA per
-// work item)
-void launch_gabor_flt(const ScaleDev* d_sd, const TileWork* d_work, int nwork, unsigned int* d_fault,
+// differentiable forward: the tile kernel on the float levels (`grid`
+// persistent CTAs)
+void launch_gabor_flt(const ScaleDev* d_sd, const TileWork* d_work, int nwork, int grid, unsigned int* d_fault,
                       cudaStream_t s, bool pipelined);
 // detection-path tile kernel that also keeps e + i o (ScaleDev::Z) for the
 // line/edge detector; one CTA per work item
@@ -111,8 +111,8 @@ void launch_detect_le(const ScaleDev* d_sd, int dataW, int dataH, const float* d
 void launch_masked_loss(const ScaleDev* d_sd, const int2* d_work, int nwork, double* d_loss, double* d_gparams,
                         cudaStream_t s);
 void launch_stencil_bwd(const ScaleDev* d_sd, const int2* d_work, int nwork, cudaStream_t s);
-// tile backward, recomputing the responses; `grid` persistent CTAs (at most
-// nwork), d_xscratch holds grid x kSpecHalf float2 (one tile spectrum per CTA)
+// tile backward, recomputing the responses; `grid` persistent CTAs,
+// d_xscratch holds grid x kSpecHalf float2 (one tile spectrum per CTA)
 void launch_gabor_bwd(const ScaleDev* d_sd, const TileWork* d_work, int nwork, int grid, float2* d_xscratch,
                       double* d_gparams, cudaStream_t s);
 
