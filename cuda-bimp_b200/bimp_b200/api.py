@@ -189,7 +189,8 @@ def getKeypoints(input, cs: CudaStuff, capacity: int = KP_MAX_POINTS, return_cou
     """
     torch = _torch()
     img = _as_gpu_u8(input)
-    kp = torch.zeros((KP_VECTOR_LENGTH, max(capacity, 1)), dtype=torch.float32, device="cuda")
+    # every column of the returned view is written by the call
+    kp = torch.empty((KP_VECTOR_LENGTH, max(capacity, 1)), dtype=torch.float32, device="cuda")
     n = C.c_int(0)
     rc = L.lib().bimp_detect_device(cs.handle, C.c_void_p(img.data_ptr()), img.stride(0),
                                     img.shape[1], img.shape[0], C.c_void_p(kp.data_ptr()),
@@ -230,20 +231,28 @@ _HOST_RECORD = np.dtype([("x", "<f4"), ("y", "<f4"), ("size", "<f4"), ("angle", 
                          ("octave", "<i4"), ("class_id", "<i4")])
 
 
+def _host_records(capacity: int):
+    """A new array for `capacity` records and its pointer: the library writes
+    the records straight into the array that the caller gets (its first part).
+    Pages that no record reaches are never touched; a zeroed ctypes array of
+    the capacity and a copy out of it took more than half of a 1080p
+    detect_host call."""
+    out = np.empty(max(capacity, 1), dtype=_HOST_RECORD)
+    return out, C.cast(out.ctypes.data, C.POINTER(L.KeyPointC))
+
+
 def detect_host(cs: CudaStuff, image: np.ndarray, capacity: int = KP_MAX_POINTS):
     """Host image in, host records out through bimp_detect_host.
 
     Returns (structured array of cv::KeyPoint fields, total count, status)."""
     img = np.ascontiguousarray(image, dtype=np.uint8)
-    out = (L.KeyPointC * max(capacity, 1))()
+    out, ptr = _host_records(capacity)
     n = C.c_int(0)
     rc = L.lib().bimp_detect_host(cs.handle, C.c_void_p(img.ctypes.data), img.strides[0], img.shape[1],
-                                  img.shape[0], out, capacity, C.byref(n), _stream_ptr())
+                                  img.shape[0], ptr, capacity, C.byref(n), _stream_ptr())
     if rc not in (L.BIMP_OK, L.BIMP_ERR_CAPACITY):
         L.check(rc, "detect_host")
-    m = min(n.value, capacity)
-    rec = np.frombuffer(out, dtype=_HOST_RECORD, count=m).copy()
-    return rec, n.value, rc
+    return out[:min(n.value, capacity)], n.value, rc
 
 
 def min_size_dims(width: int, height: int) -> tuple:
@@ -408,7 +417,6 @@ class Pipeline:
         self._h = h
         self.width, self.height, self.depth, self.capacity = int(width), int(height), int(depth), int(capacity)
         self._frames = []
-        self._out = (L.KeyPointC * self.capacity)()
 
     def in_flight(self) -> int:
         return int(L.lib().bimp_pipeline_in_flight(self._h))
@@ -424,14 +432,13 @@ class Pipeline:
     def pop(self, capacity: int | None = None):
         """(records, total, status) of the oldest frame in flight."""
         cap = self.capacity if capacity is None else int(capacity)
+        out, ptr = _host_records(min(cap, self.capacity))
         n = C.c_int(0)
-        rc = L.lib().bimp_pipeline_pop(self._h, self._out, cap, C.byref(n))
+        rc = L.lib().bimp_pipeline_pop(self._h, ptr, cap, C.byref(n))
         if rc not in (L.BIMP_OK, L.BIMP_ERR_CAPACITY):
             L.check(rc, "pipeline_pop")
         self._frames.pop(0)
-        m = min(n.value, cap, self.capacity)
-        rec = np.frombuffer(self._out, dtype=_HOST_RECORD, count=m).copy()
-        return rec, n.value, rc
+        return out[:min(n.value, cap, self.capacity)], n.value, rc
 
     def close(self):
         if getattr(self, "_h", None) is not None:
@@ -468,6 +475,14 @@ class Batch:
             pitch = C.c_size_t()
             L.check(L.lib().bimp_batch_image(h, i, C.byref(ptr), C.byref(pitch)), "batch_image")
             self._inputs.append((ptr.value, pitch.value))
+        # aliases of the library's input and keypoint buffers, made once
+        self._input_tensors = [_wrap_device(p, (hh, w), (pitch, 1), "|u1")
+                               for (p, pitch), (w, hh) in zip(self._inputs, self.sizes)]
+        self._kp = []
+        for i in range(n):
+            ptr, ld = C.c_void_p(), C.c_size_t()
+            L.check(L.lib().bimp_batch_keypoints_device(h, i, C.byref(ptr), C.byref(ld)), "batch_keypoints")
+            self._kp.append(_wrap_device(ptr.value, (KP_VECTOR_LENGTH, ld.value), (4 * ld.value, 4), "<f4"))
         self._counts = torch.zeros(n, dtype=torch.int32, device="cuda")
 
     def input_view(self, i: int):
@@ -476,9 +491,7 @@ class Batch:
 
     def input_tensor(self, i: int):
         """uint8 CUDA tensor (h x w, row stride = pitch) aliasing image i's input."""
-        ptr, pitch = self._inputs[i]
-        w, h = self.sizes[i]
-        return _wrap_device(ptr, (h, w), (pitch, 1), "|u1")
+        return self._input_tensors[i]
 
     def load(self, images, stream=None):
         """Copy uint8 images (numpy or CUDA tensors) into the batch inputs."""
@@ -531,16 +544,11 @@ class Batch:
         return out
 
     def keypoints(self, i: int):
-        torch = _torch()
-        ptr = C.c_void_p()
-        ld = C.c_size_t()
-        L.check(L.lib().bimp_batch_keypoints_device(self._h, i, C.byref(ptr), C.byref(ld)),
-                "batch_keypoints")
-        n = int(self.counts()[i].item())
-        n = min(n, self.kp_capacity)
-        # wrap the internal matrix without copying
-        buf = _wrap_device(ptr.value, (KP_VECTOR_LENGTH, ld.value), (4 * ld.value, 4), "<f4")
-        return buf[:, :n]
+        """View of image i's internal keypoint matrix (not copied), as many
+        columns as the last run found (waits for it)."""
+        n = C.c_int(0)
+        L.check(L.lib().bimp_batch_count(self._h, int(i), C.byref(n), _stream_ptr()), "batch_keypoints")
+        return self._kp[i][:, :min(n.value, self.kp_capacity)]
 
     def close(self):
         if getattr(self, "_h", None) is not None:

@@ -427,10 +427,10 @@ struct Engine {
     const size_t offSten = a.reserve(sizeof(int2) * std::max<size_t>(1, sten.size()));
     const size_t offRows = a.reserve(sizeof(int2) * std::max<size_t>(1, rows.size()));
     const size_t offNmsCtas = a.reserve(sizeof(NmsCta) * std::max<size_t>(1, nmsCtas.size()));
-    const size_t offTotals = a.reserve(sizeof(int) * n);
-    // per-detection reset region: the map maxima and the fault word
+    // per-detection reset region: the map maxima and the fault word; the
+    // keypoint totals follow the fault word, so that one copy brings both back
     resetBytes = sizeof(unsigned int) * (sds.size() + 1);
-    const size_t offMax = a.reserve(resetBytes);
+    const size_t offMax = a.reserve(resetBytes + sizeof(int) * n);
     const size_t offNmsCount = a.reserve(sizeof(int) * std::max<size_t>(1, nmsCtas.size()));
     const size_t offOuts = a.reserve(sizeof(KpOut) * n);
     const size_t offPyr = a.reserve(sizeof(PyrJob) * std::max<size_t>(1, h_pyr.size()));
@@ -488,8 +488,8 @@ struct Engine {
     d_sten = reinterpret_cast<int2*>(base + offSten);
     d_rows = reinterpret_cast<int2*>(base + offRows);
     d_nmsCtas = reinterpret_cast<NmsCta*>(base + offNmsCtas);
-    d_totals = reinterpret_cast<int*>(base + offTotals);
     d_maxKeys = reinterpret_cast<unsigned int*>(base + offMax);
+    d_totals = reinterpret_cast<int*>(base + offMax + resetBytes);
     d_nmsCount = reinterpret_cast<int*>(base + offNmsCount);
     d_fault = d_maxKeys + sds.size();
     d_outs = reinterpret_cast<KpOut*>(base + offOuts);
@@ -589,7 +589,7 @@ struct bimp_context {
   std::vector<ScaleHost> info;
   // host path: pinned count/fault words; device scratch the NMS writes
   // cv::KeyPoint records into before the single copy to the caller's array
-  int* h_count = nullptr;   // pinned: [0] keypoint total, [1] device fault word
+  int* h_count = nullptr;   // pinned: [0] device fault word, [1] keypoint total
   float* d_kpScratch = nullptr;
   int d_kpScratchCap = 0;
   // pinned host staging of the records, and how many records go back with
@@ -621,7 +621,7 @@ struct bimp_batch {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   cudaStream_t capStream = nullptr;
-  int* h_totals = nullptr;   // pinned: n_images totals, then the device fault word
+  int* h_totals = nullptr;   // pinned: the device fault word, then n_images totals
   std::vector<bimp_keypoint> tmp;
 };
 
@@ -838,11 +838,10 @@ int bimp_detect_device(bimp_context* c, const uint8_t* d_image, size_t pitch, in
   int rc = ctx_run(c, d_image, pitch, width, height, cudaMemcpyDeviceToDevice, d_kp, ld, capacity,
                    nullptr, s);
   if (rc != BIMP_OK) return rc;
-  BIMP_CUDA(cudaMemcpyAsync(c->h_count, c->eng.d_totals, sizeof(int), cudaMemcpyDeviceToHost, s));
-  BIMP_CUDA(cudaMemcpyAsync(c->h_count + 1, c->eng.d_fault, sizeof(int), cudaMemcpyDeviceToHost, s));
+  BIMP_CUDA(cudaMemcpyAsync(c->h_count, c->eng.d_fault, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
   BIMP_CUDA(cudaStreamSynchronize(s));
-  *n_found = *c->h_count;
-  if (c->h_count[1]) return fail(BIMP_ERR_CUDA, "a bounded device wait expired in the tile kernel");
+  *n_found = c->h_count[1];
+  if (c->h_count[0]) return fail(BIMP_ERR_CUDA, "a bounded device wait expired in the tile kernel");
   if (*n_found > capacity)
     return fail(BIMP_ERR_CAPACITY, "keypoints exceed capacity (" + std::to_string(*n_found) + ")");
   return BIMP_OK;
@@ -878,8 +877,7 @@ static int host_enqueue(bimp_context* c, const uint8_t* image, size_t pitch, int
   if (rc != BIMP_OK) return rc;
   rc = ctx_run(c, image, pitch, width, height, cudaMemcpyHostToDevice, c->d_kpScratch, cap, capacity, nullptr, s, 1);
   if (rc != BIMP_OK) return rc;
-  BIMP_CUDA(cudaMemcpyAsync(c->h_count, c->eng.d_totals, sizeof(int), cudaMemcpyDeviceToHost, s));
-  BIMP_CUDA(cudaMemcpyAsync(c->h_count + 1, c->eng.d_fault, sizeof(int), cudaMemcpyDeviceToHost, s));
+  BIMP_CUDA(cudaMemcpyAsync(c->h_count, c->eng.d_fault, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
   *spec = std::min(capacity, c->specRecords);
   if (*spec > 0)
     BIMP_CUDA(cudaMemcpyAsync(c->h_stage, c->d_kpScratch, sizeof(bimp_keypoint) * (size_t)*spec,
@@ -892,9 +890,9 @@ static int host_enqueue(bimp_context* c, const uint8_t* image, size_t pitch, int
 // come back with one more copy and synchronisation, then everything is
 // copied from the staging into the caller's array.
 static int host_finish(bimp_context* c, int spec, bimp_keypoint* out, int capacity, int* n_found, cudaStream_t s) {
-  const int total = c->h_count[0];
+  const int total = c->h_count[1];
   *n_found = total;
-  if (c->h_count[1]) return fail(BIMP_ERR_CUDA, "a bounded device wait expired");
+  if (c->h_count[0]) return fail(BIMP_ERR_CUDA, "a bounded device wait expired");
   const int n = std::min(total, capacity);
   if (n > spec) {
     BIMP_CUDA(cudaMemcpyAsync(c->h_stage + spec, reinterpret_cast<const bimp_keypoint*>(c->d_kpScratch) + spec,
@@ -1179,6 +1177,16 @@ int bimp_batch_counts(bimp_batch* b, int* d_counts, void* stream) {
   return BIMP_OK;
 }
 
+int bimp_batch_count(bimp_batch* b, int i, int* n_found, void* stream) {
+  if (!b || !n_found || i < 0 || i >= b->eng.nImages) return fail(BIMP_ERR_INVALID, "bad batch count arguments");
+  BIMP_CUDA(cudaSetDevice(b->eng.device));
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  BIMP_CUDA(cudaMemcpyAsync(b->h_totals + 1 + i, b->eng.d_totals + i, sizeof(int), cudaMemcpyDeviceToHost, s));
+  BIMP_CUDA(cudaStreamSynchronize(s));
+  *n_found = b->h_totals[1 + i];
+  return BIMP_OK;
+}
+
 int bimp_batch_scale_info(const bimp_batch* b, int i, int scale, bimp_scale_info* out) {
   if (!b || !out || i < 0 || i >= b->eng.nImages || scale < 0 || scale >= b->eng.nScales)
     return fail(BIMP_ERR_INVALID, "bad batch scale index");
@@ -1228,13 +1236,12 @@ int bimp_batch_detect_host(bimp_batch* b, const uint8_t* const* images, const si
                                 e.heights[i], cudaMemcpyHostToDevice, s));
   }
   BIMP_CUDA(cudaGraphLaunch(b->exec, s));
-  BIMP_CUDA(cudaMemcpyAsync(b->h_totals, e.d_totals, sizeof(int) * e.nImages, cudaMemcpyDeviceToHost, s));
-  BIMP_CUDA(cudaMemcpyAsync(b->h_totals + e.nImages, e.d_fault, sizeof(int), cudaMemcpyDeviceToHost, s));
+  BIMP_CUDA(cudaMemcpyAsync(b->h_totals, e.d_fault, sizeof(int) * (1 + e.nImages), cudaMemcpyDeviceToHost, s));
   BIMP_CUDA(cudaStreamSynchronize(s));
-  if (b->h_totals[e.nImages]) return fail(BIMP_ERR_CUDA, "a bounded device wait expired in the tile kernel");
+  if (b->h_totals[0]) return fail(BIMP_ERR_CUDA, "a bounded device wait expired in the tile kernel");
   int status = BIMP_OK;
   for (int i = 0; i < e.nImages; ++i) {
-    n_found[i] = b->h_totals[i];
+    n_found[i] = b->h_totals[1 + i];
     const int cap = std::min(capacities ? capacities[i] : 0, e.kpCapInternal);
     const int n = std::min(n_found[i], cap);
     if (n_found[i] > cap) status = BIMP_ERR_CAPACITY;

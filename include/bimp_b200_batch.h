@@ -81,6 +81,9 @@ int bimp_batch_run(bimp_batch* batch, void* stream);
 /* Copies the per-image keypoint totals (n_images ints) to device memory. */
 int bimp_batch_counts(bimp_batch* batch, int* d_counts, void* stream);
 
+/* Keypoint total of image i to host memory; waits for `stream`. */
+int bimp_batch_count(bimp_batch* batch, int i, int* n_found, void* stream);
+
 /* Internal 7 x ld keypoint matrix of image i, (scale, y, x) order; only the
  * first min(count, ld) columns are written. */
 int bimp_batch_keypoints_device(bimp_batch* batch, int i, const float** d_kp, size_t* ld);
