@@ -128,6 +128,7 @@ struct Engine {
   int nWork = 0;                  // entries of the work list
   int2* d_sten = nullptr;
   int nSten = 0;
+  std::vector<int> stenStart;     // per entry (and the end): its first block in d_sten
   int2* d_rows = nullptr;
   int nRows = 0;
   NmsCta* d_nmsCtas = nullptr;          // the NMS kernels' row groups (one image each)
@@ -343,6 +344,7 @@ struct Engine {
         d.rowBase = static_cast<int>(rows.size());
         for (int tIdx = 0; tIdx < d.tilesX * d.tilesY; ++tIdx) tiles.push_back({entry, tIdx});
         const int nbx = (s.dataW + 31) / 32, nby = (s.dataH + kStencilBlockH - 1) / kStencilBlockH;
+        stenStart.push_back(static_cast<int>(sten.size()));
         for (int b = 0; b < nbx * nby; ++b) sten.push_back(make_int2(entry, b));
         const int yEnd = std::min(s.dataH - s.off - 1, s.dataH - 2);
         // keypoint-decision words: 32-pixel-aligned words covering a row's
@@ -403,6 +405,7 @@ struct Engine {
     nWork = static_cast<int>(work.size());
     tileGridReq = std::max(0, defGrid);
     nSten = static_cast<int>(sten.size());
+    stenStart.push_back(nSten);
     nRows = static_cast<int>(rows.size());
     const size_t offSd = a.reserve(sizeof(ScaleDev) * sds.size());
     {   // the tile buffer holds the largest plan the autotuner may choose
@@ -929,9 +932,11 @@ int bimp_dense_map(bimp_context* c, int scale, int which, float* d_out, size_t l
   if (which == 1) {
     // S is not on the keypoint path: detection writes D only, and the
     // single-stopped map is computed here from the last detection's complex
-    // cells (the same stencil pass, which rewrites D with identical values)
-    if (c->eng.nSten > 0)
-      launch_stencil(c->eng.d_sd, c->eng.d_sten, c->eng.nSten, c->eng.d_fault, s, kStencilDS);
+    // cells (the same stencil pass over this scale's blocks, which rewrites D
+    // with identical values; over every scale's, the nine scales of a VGA
+    // image's responses took nine times 20 us)
+    const int b0 = c->eng.stenStart[scale], b1 = c->eng.stenStart[scale + 1];
+    launch_stencil(c->eng.d_sd, c->eng.d_sten + b0, b1 - b0, c->eng.d_fault, s, kStencilDS);
     BIMP_CUDA(cudaGetLastError());
   }
   const float* src = which == 0 ? d.D : d.S;
