@@ -4,8 +4,7 @@
 //
 // Nothing of the responses survives the forward: the backward recomputes each
 // tile's spectrum and e + i o.  The per-cell scratch (complex cells C and
-// their gradient, the inhibition maps T and R) exists for a chunk of images
-// at a time; the forward and the backward walk the chunks in order, and the
+// their gradient) exists for a chunk of images at a time; the forward and the backward walk the chunks in order, and the
 // entries of images in different chunks share the same scratch.
 #include <cuda_runtime.h>
 
@@ -160,15 +159,14 @@ struct bimp_adjoint {
     std::vector<int2> sten, stenB;
     std::vector<ScaleDev> sds;
     std::vector<size_t> offD, offBits;                  // per entry
-    std::vector<size_t> offC, offT, offR, offGC, offGW;  // per (chunk slot, scale)
+    std::vector<size_t> offC, offGC, offGW;  // per (chunk slot, scale)
     // images per chunk: all of them while their per-cell scratch stays under
     // kChunkBudget (BIMP_ADJOINT_CHUNK overrides it, for tests)
     {
       size_t per = 0;
       for (const ScaleHost& sc : geo) {
         const size_t cStride = (size_t)(sc.dataH + 2) * up(sc.dataW + 1, 32);
-        per += 2 * sizeof(float) * kNumOri * cStride + sizeof(float) * kNumOri * (sc.dataH + 1) +
-               2 * sizeof(float) * (size_t)sc.dataH * up(sc.dataW, 32);
+        per += 2 * sizeof(float) * kNumOri * cStride + sizeof(float) * kNumOri * (sc.dataH + 1);
       }
       constexpr size_t kChunkBudget = size_t(8) << 30;
       chunk = static_cast<int>(std::max<size_t>(1, std::min<size_t>(n, kChunkBudget / std::max<size_t>(per, 1))));
@@ -180,12 +178,9 @@ struct bimp_adjoint {
     for (int k = 0; k < chunk; ++k) {
       for (const ScaleHost& sc : geo) {
         const size_t cStride = (size_t)(sc.dataH + 2) * up(sc.dataW + 1, 32);
-        const size_t mapB = sizeof(float) * (size_t)sc.dataH * up(sc.dataW, 32);
         offC.push_back(take(sizeof(float) * kNumOri * cStride));
         offGC.push_back(take(sizeof(float) * kNumOri * cStride));
         offGW.push_back(take(sizeof(float) * kNumOri * (sc.dataH + 1)));
-        offT.push_back(take(mapB));
-        offR.push_back(take(mapB));
       }
     }
     for (int i = 0; i < n; ++i) {
@@ -309,8 +304,6 @@ struct bimp_adjoint {
       d.Z = nullptr;
       d.gC = reinterpret_cast<float*>(b + offGC[slot]);
       d.gWrap = reinterpret_cast<float*>(b + offGW[slot]);
-      d.T = reinterpret_cast<float*>(b + offT[slot]);
-      d.R = reinterpret_cast<float*>(b + offR[slot]);
       d.D = reinterpret_cast<float*>(b + offD[e2]);
       d.bits = reinterpret_cast<unsigned int*>(b + offBits[e2]);
       d.M = d_M + (size_t)i * maskStride + maskOff[si];
@@ -384,8 +377,8 @@ struct bimp_adjoint {
       const int i1 = std::min(n, i0 + chunk);
       const Plan& p = fwdPlan[i0 / chunk];
       launch_gabor_flt(d_sd, d_tiles + p.first, p.items, p.grid, fault, s, pipelined);
-      launch_stencil(d_sd, d_sten + stenStart[i0], stenStart[i1] - stenStart[i0], fault, s, kStencilAdj);
-      launch_masked_loss(d_sd, d_sten + stenStart[i0], stenStart[i1] - stenStart[i0], d_loss, d_gp, s);
+      launch_stencil(d_sd, d_sten + stenStart[i0], stenStart[i1] - stenStart[i0], fault, s, kStencilAdj, false, d_loss,
+                     d_gp);
     }
     if (loss) ADJ_CUDA(cudaMemcpyAsync(loss, d_loss, sizeof(double), cudaMemcpyDeviceToDevice, s));
     ADJ_CUDA(cudaGetLastError());

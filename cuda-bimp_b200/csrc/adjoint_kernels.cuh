@@ -3,7 +3,6 @@
 //
 //   k_pyr_down_f        float pyramid level (pyrDown without uint8 rounding)
 //   k_pyr_down_f_adj    its transpose (scatter-add of the 5x5 taps)
-//   k_masked_loss       sum M * D (the loss) and the w_tan / w_rad gradients
 //   k_stencil_bwd       gather form of d L / d C over the stencil window from
 //                       the ReLU states the forward stencil recorded (when
 //                       fftW == dataW, window column dataW is the torus
@@ -74,39 +73,6 @@ __device__ __forceinline__ void block_add_double(double v, double* dst) {
   }
 }
 
-// Over the forward stencil blocks (32 x kStencilBlockH pixels, the forward
-// stencil's block list), a persistent grid: sum M * D into loss[0], and
-// -sum M * T, -sum M * R (dL/dw_tan and dL/dw_rad: D = D0 - w_tan T -
-// w_rad R) into gparams[2..3].  Each CTA accumulates its blocks in registers
-// and adds once per quantity (a per-block atomic on the same three words
-// serialises).
-__global__ void __launch_bounds__(256) k_masked_loss(const ScaleDev* __restrict__ sds, const int2* __restrict__ work,
-                                                     int nwork, double* __restrict__ loss,
-                                                     double* __restrict__ gparams) {
-  double acc = 0.0, accT = 0.0, accR = 0.0;
-  for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
-    const int2 item = work[w];
-    const ScaleDev* sd = sds + item.x;
-    const int W = sd->dataW, H = sd->dataH;
-    const int nbx = (W + kStX - 1) / kStX;
-    const int by = item.y / nbx, bx = item.y - by * nbx;
-    const int x = bx * kStX + (threadIdx.x & 31);
-    for (int i = threadIdx.x >> 5; i < kStencilBlockH; i += 8) {
-      const int y = by * kStencilBlockH + i;
-      if (x < W && y < H) {
-        const double m = sd->M[(size_t)y * W + x];
-        const size_t k = (size_t)y * sd->dPitch + x;
-        acc += m * (double)sd->D[k];
-        accT += m * (double)sd->T[k];
-        accR += m * (double)sd->R[k];
-      }
-    }
-  }
-  block_add_double(acc, loss);
-  block_add_double(-accT, gparams + 2);
-  block_add_double(-accR, gparams + 3);
-}
-
 // --- stencil backward ------------------------------------------------------
 constexpr int kBwQW = kStX + 2 * kHalo;        // 48: source pixels +-8 around the block
 constexpr int kStBwThreads = 256;
@@ -116,7 +82,7 @@ constexpr int kStBwThreads = 256;
 // contributes its loss weight M(q) times the ReLU state the forward recorded
 // at q (ScaleDev::bits).  Sources lie within +-8 of p.  The tangential and
 // radial weights are constants here; their own gradients come from
-// k_masked_loss.
+// the forward stencil.
 __global__ void __launch_bounds__(kStBwThreads)
 k_stencil_bwd(const ScaleDev* __restrict__ sds, const int2* __restrict__ work) {
   __shared__ float sM[kBwQW * kBwQW];

@@ -73,8 +73,6 @@ struct ScaleDev {
   float* gC;              // d loss / d complex cell, C layout
   float* gWrap;           // fftW == dataW: d loss / d window (r, dataW), kNumOri x (dataH + 1)
   float* gLvl;            // d loss / d float level, lvlPitchF floats per row
-  float* T;               // tangential inhibition map, dataH x dPitch
-  float* R;               // radial inhibition map, dataH x dPitch
   unsigned int* bits;     // ReLU states, 4 bits per orientation, dataH x dPitch
   const float4* bwA;      // per orientation, kSpecHalf entries {G(k), G(-k), dGa(k), dGr(k)}
   const float2* bwB;      //   {dGa(-k), dGr(-k)}; dG* = spectra of d taps / d alpha, d rho

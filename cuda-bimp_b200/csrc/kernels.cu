@@ -290,8 +290,8 @@ __device__ __forceinline__ int soff(const StencilPar& P, int k, int o) {
 // one float rounding apart).
 // Stencil modes: detection writes D only (the single-stopped map S is not on
 // the keypoint path); responses write D and S; the differentiable forward
-// writes D, the tangential and radial sums T, R and the ReLU states the
-// adjoint needs: per orientation o, bit 4o double-stopped d > 0, 4o+1
+// writes D and the ReLU states the adjoint needs and sums M * D, M * T, M * R
+// (T, R: the tangential and radial inhibition): per orientation o, bit 4o double-stopped d > 0, 4o+1
 // tangential t > 0, 4o+2 radial r > 0, 4o+3 the first radial term r1 > 0
 // (all 0 where the bounds test fails).
 // Whether orientation o's taps at offsets k, k + 1 (0: end-stopping,
@@ -435,10 +435,16 @@ __device__ __forceinline__ void stencil_pair_d(const float* __restrict__ s_c, in
 struct StencilOut {
   float* D;
   float* S;
-  float* T;
-  float* R;
+  const float* M;
   unsigned int* bits;
   int pitch;
+};
+
+// A thread's share of the differentiable forward's sums over its pixels:
+// M * D (the loss) and M * T, M * R (dL/dw_tan and dL/dw_rad with the sign
+// changed: D = D0 - w_tan T - w_rad R).
+struct StencilSums {
+  double l = 0.0, t = 0.0, r = 0.0;
 };
 
 // The rows of one thread (ly0, ly0 + NT/32, ...).  CHECK = false: every
@@ -446,13 +452,21 @@ struct StencilOut {
 // the rows run as straight-line code whose loads and sums interleave.
 template <bool CHECK, int PAT, int MODE, int NT>
 __device__ __forceinline__ float stencil_rows(const float* __restrict__ s_c, const StencilPar& P, int x0, int y0,
-                                              int W, int H, float gain, float wT, float wR, const StencilOut& out) {
+                                              int W, int H, float gain, float wT, float wR, const StencilOut& out,
+                                              StencilSums& sums) {
   const int t = threadIdx.x;
   const int lx = t & 31, ly0 = t >> 5;
   const int x = x0 + lx;
   constexpr int kRows = kFwY / (NT / 32);
-  float D[kRows], S[kRows], T[kRows], R[kRows];
+  float D[kRows], S[kRows], T[kRows], R[kRows], M[kRows];
   unsigned int b[kRows];
+  if constexpr (MODE == kStencilAdj) {   // loaded ahead of the arithmetic
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) {
+      const int y = y0 + ly0 + (NT / 32) * i;
+      M[i] = !CHECK || (x < W && y < H) ? __ldg(out.M + (size_t)y * W + x) : 0.f;
+    }
+  }
   if constexpr (!CHECK && PAT > 0 && MODE == kStencilD && NT / 32 == 16) {
 #pragma unroll
     for (int i = 0; i < kRows; i += 2)
@@ -474,9 +488,11 @@ __device__ __forceinline__ float stencil_rows(const float* __restrict__ s_c, con
     out.D[k] = D[i];
     if constexpr (MODE == kStencilDS) out.S[k] = S[i];
     if constexpr (MODE == kStencilAdj) {
-      out.T[k] = T[i];
-      out.R[k] = R[i];
       out.bits[k] = b[i];
+      const double m = M[i];
+      sums.l += m * (double)D[i];
+      sums.t += m * (double)T[i];
+      sums.r += m * (double)R[i];
     }
     dmax = fmaxf(dmax, D[i]);
   }
@@ -485,11 +501,12 @@ __device__ __forceinline__ float stencil_rows(const float* __restrict__ s_c, con
 
 template <int PAT, int MODE, int NT>
 __device__ __forceinline__ float stencil_block(const float* __restrict__ s_c, const StencilPar& P, int x0, int y0,
-                                               int W, int H, float gain, float wT, float wR, const StencilOut& out) {
+                                               int W, int H, float gain, float wT, float wR, const StencilOut& out,
+                                               StencilSums& sums) {
   // no bounds test needed when every pixel of the block is >= 8 from the edges
   const bool inner = x0 >= kHalo && x0 + kStX <= W - kHalo && y0 >= kHalo && y0 + kFwY <= H - kHalo;
-  return inner ? stencil_rows<false, PAT, MODE, NT>(s_c, P, x0, y0, W, H, gain, wT, wR, out)
-               : stencil_rows<true, PAT, MODE, NT>(s_c, P, x0, y0, W, H, gain, wT, wR, out);
+  return inner ? stencil_rows<false, PAT, MODE, NT>(s_c, P, x0, y0, W, H, gain, wT, wR, out, sums)
+               : stencil_rows<true, PAT, MODE, NT>(s_c, P, x0, y0, W, H, gain, wT, wR, out, sums);
 }
 
 // Persistent, warp-specialised stencil kernel: one CTA per SM walks the block
@@ -526,7 +543,8 @@ struct StencilPre {
   int e1, e2, i1, i2, h1, h2;
   int pattern, pitch;
   float gain, wT, wR;
-  float *D, *S, *T, *R;
+  float *D, *S;
+  const float* M;
   unsigned int *bits, *maxKey;
   const void* cMap;
 };
@@ -549,7 +567,7 @@ __device__ __forceinline__ StencilPre stencil_fetch(const ScaleDev* __restrict__
   if (lane == kNumOri) {
     r.pattern = sd->pattern; r.pitch = sd->dPitch;
     r.gain = sd->radialGain; r.wT = sd->wTan; r.wR = sd->wRad;
-    r.D = sd->D; r.S = sd->S; r.T = sd->T; r.R = sd->R; r.bits = sd->bits; r.maxKey = sd->maxKey;
+    r.D = sd->D; r.S = sd->S; r.M = sd->M; r.bits = sd->bits; r.maxKey = sd->maxKey;
   }
   if (lane == 0) r.cMap = sd->cMap;
   return r;
@@ -570,7 +588,7 @@ __device__ __forceinline__ void stencil_put(const StencilPre& r, StencilBlk& B, 
   } else if (lane == kNumOri) {
     B.x0 = r.x0; B.y0 = r.y0; B.W = W; B.H = H; B.pattern = r.pattern;
     B.gain = r.gain; B.wT = r.wT; B.wR = r.wR;
-    B.out.D = r.D; B.out.S = r.S; B.out.T = r.T; B.out.R = r.R; B.out.bits = r.bits;
+    B.out.D = r.D; B.out.S = r.S; B.out.M = r.M; B.out.bits = r.bits;
     B.out.pitch = r.pitch;
     B.maxKey = r.maxKey;
   }
@@ -594,7 +612,7 @@ __device__ __forceinline__ void stencil_stage_tma(const void* cMap, int x0, int 
 template <int MODE>
 __global__ void __launch_bounds__(kStThreads, kStCtasPerSm)
 k_stencil(const ScaleDev* __restrict__ sds, const int2* __restrict__ work, int nwork,
-          unsigned int* __restrict__ fault_word) {
+          unsigned int* __restrict__ fault_word, double* __restrict__ loss, double* __restrict__ gparams) {
   extern __shared__ float4 s_c4[];   // kStBufs buffers of kNumOri x kStH x kStW floats (+128 B for alignment)
   // TMA box destinations are 128-byte aligned.  The offset is added to the
   // shared-memory pointer itself (not through an integer round trip), so
@@ -647,6 +665,7 @@ k_stencil(const ScaleDev* __restrict__ sds, const int2* __restrict__ work, int n
   // one per block: consecutive blocks share their scale's max word).
   unsigned int* runKey = nullptr;
   float runMax = -INFINITY;
+  StencilSums sums;
   auto flush = [&]() {
     float m = runMax;
 #pragma unroll
@@ -668,16 +687,35 @@ k_stencil(const ScaleDev* __restrict__ sds, const int2* __restrict__ work, int n
     }
     float dmax;
     if (B.pattern == 1)
-      dmax = stencil_block<1, MODE, kStConsumers>(s_c, B.P, B.x0, B.y0, B.W, B.H, B.gain, B.wT, B.wR, B.out);
+      dmax = stencil_block<1, MODE, kStConsumers>(s_c, B.P, B.x0, B.y0, B.W, B.H, B.gain, B.wT, B.wR, B.out, sums);
     else if (B.pattern == 2)
-      dmax = stencil_block<2, MODE, kStConsumers>(s_c, B.P, B.x0, B.y0, B.W, B.H, B.gain, B.wT, B.wR, B.out);
+      dmax = stencil_block<2, MODE, kStConsumers>(s_c, B.P, B.x0, B.y0, B.W, B.H, B.gain, B.wT, B.wR, B.out, sums);
     else
-      dmax = stencil_block<0, MODE, kStConsumers>(s_c, B.P, B.x0, B.y0, B.W, B.H, B.gain, B.wT, B.wR, B.out);
+      dmax = stencil_block<0, MODE, kStConsumers>(s_c, B.P, B.x0, B.y0, B.W, B.H, B.gain, B.wT, B.wR, B.out, sums);
     runMax = fmaxf(runMax, dmax);
     __syncwarp();
     if (lane == 0) mbar_arrive(empty0 + 8 * b);   // this warp is done with buffer b and blk[b]
   }
   flush();
+  if constexpr (MODE == kStencilAdj) {
+    // the loss and the w_tan / w_rad gradients: one addition per CTA and sum
+    // (in a kernel of their own, reading D, T and R back, these took 69 us of
+    // 16 x 512 x 512 with 6 scales)
+    __shared__ double s_sum[3][kStConsumers / 32];
+    double v[3] = {sums.l, -sums.t, -sums.r};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+#pragma unroll
+      for (int sh = 16; sh > 0; sh >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], sh);
+      if (lane == 0) s_sum[k][warp] = v[k];
+    }
+    named_barrier(1, kStConsumers);
+    if (t < 3) {
+      double a = 0.0;
+      for (int k = 0; k < kStConsumers / 32; ++k) a += s_sum[t][k];
+      atomicAdd(t == 0 ? loss : gparams + 1 + t, a);
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1347,10 +1385,6 @@ void launch_pyr_f_adj(const PyrJobF* d_jobs, int njobs, int maxW, int maxH, cuda
   dim3 b(32, 8), g((maxW + 31) / 32, (maxH + 7) / 8, njobs);
   k_pyr_down_f_adj<<<g, b, 0, s>>>(d_jobs);
 }
-void launch_masked_loss(const ScaleDev* d_sd, const int2* d_work, int nwork, double* d_loss, double* d_gparams,
-                        cudaStream_t s) {
-  if (nwork > 0) k_masked_loss<<<std::min(nwork, 4 * num_sms()), 256, 0, s>>>(d_sd, d_work, nwork, d_loss, d_gparams);
-}
 void launch_stencil_bwd(const ScaleDev* d_sd, const int2* d_work, int nwork, cudaStream_t s) {
   if (nwork > 0) k_stencil_bwd<<<nwork, kStBwThreads, 0, s>>>(d_sd, d_work);
 }
@@ -1362,15 +1396,18 @@ void launch_gabor_bwd(const ScaleDev* d_sd, const TileWork* d_work, int nwork, i
                                                                                  d_gparams);
 }
 void launch_stencil(const ScaleDev* d_sd, const int2* d_work, int nwork, unsigned int* d_fault, cudaStream_t s,
-                    int mode, bool pdl) {
+                    int mode, bool pdl, double* d_loss, double* d_gparams) {
   if (nwork <= 0) return;
   const int grid = std::min(nwork, kStCtasPerSm * num_sms());
   if (mode == kStencilDS)
-    launch_ex(k_stencil<kStencilDS>, grid, kStThreads, stencil_smem_bytes(), s, pdl, d_sd, d_work, nwork, d_fault);
+    launch_ex(k_stencil<kStencilDS>, grid, kStThreads, stencil_smem_bytes(), s, pdl, d_sd, d_work, nwork, d_fault,
+              d_loss, d_gparams);
   else if (mode == kStencilAdj)
-    launch_ex(k_stencil<kStencilAdj>, grid, kStThreads, stencil_smem_bytes(), s, pdl, d_sd, d_work, nwork, d_fault);
+    launch_ex(k_stencil<kStencilAdj>, grid, kStThreads, stencil_smem_bytes(), s, pdl, d_sd, d_work, nwork, d_fault,
+              d_loss, d_gparams);
   else
-    launch_ex(k_stencil<kStencilD>, grid, kStThreads, stencil_smem_bytes(), s, pdl, d_sd, d_work, nwork, d_fault);
+    launch_ex(k_stencil<kStencilD>, grid, kStThreads, stencil_smem_bytes(), s, pdl, d_sd, d_work, nwork, d_fault,
+              d_loss, d_gparams);
 }
 void launch_nms_two_pass(const ScaleDev* d_sd, const int2* d_rows, const NmsCta* d_ctas, int nctas, int* d_ctaCount,
                          int* d_totals, const KpOut* d_outs, cudaStream_t s, bool pdl) {

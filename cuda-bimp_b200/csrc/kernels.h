@@ -71,12 +71,13 @@ struct alignas(64) TensorMapBlob {
 bool encode_c_maps(const ScaleDev* sds, int n, void* maps, std::string& err);
 
 // Stencil output modes: D only (detection), D and S (responses), and the
-// differentiable forward (D, T, R, ReLU states).
+// differentiable forward (D, ReLU states; adds sum M * D to d_loss[0] and
+// -sum M * T, -sum M * R to d_gparams[2..3]).
 enum StencilMode { kStencilD = 0, kStencilDS = 1, kStencilAdj = 2 };
 // Persistent stencil (one CTA per SM); an expired staging wait sets bit 1 of
 // *d_fault.
 void launch_stencil(const ScaleDev* d_sd, const int2* d_work, int nwork, unsigned int* d_fault, cudaStream_t s,
-                    int mode = kStencilD, bool pdl = false);
+                    int mode = kStencilD, bool pdl = false, double* d_loss = nullptr, double* d_gparams = nullptr);
 // NMS in two launches (k_nms_decide, k_nms_emit): one CTA per group of up to
 // kNmsRowsPerCta candidate rows of one image; d_ctaCount holds nctas ints
 // (written by the first kernel, read by the second).
@@ -108,8 +109,6 @@ void launch_gabor_keep_z(const ScaleDev* d_sd, const TileWork* d_work, int nwork
 // line/edge detection on one scale (d_sd: that scale's descriptor, with Z)
 void launch_detect_le(const ScaleDev* d_sd, int dataW, int dataH, const float* d_ch, int chLd, float* d_result,
                       float* d_ori, int8_t* d_type, int ld, cudaStream_t s);
-void launch_masked_loss(const ScaleDev* d_sd, const int2* d_work, int nwork, double* d_loss, double* d_gparams,
-                        cudaStream_t s);
 void launch_stencil_bwd(const ScaleDev* d_sd, const int2* d_work, int nwork, cudaStream_t s);
 // tile backward, recomputing the responses; `grid` persistent CTAs,
 // d_xscratch holds grid x kSpecHalf float2 (one tile spectrum per CTA)
