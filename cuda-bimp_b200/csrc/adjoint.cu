@@ -396,7 +396,7 @@ struct bimp_adjoint {
       const Plan& p = bwdPlan[i0 / chunk];
       launch_gabor_bwd(d_sd, d_tiles + p.first, p.items, p.grid, d_xscr, d_gp, s);
     }
-    for (int l = maxLevel; l >= 1; --l) launch_pyr_f_adj(d_pyrAdj + (l - 1) * n, n, lw[l], lh[l], s);
+    for (int l = maxLevel; l >= 1; --l) launch_pyr_f_adj(d_pyrAdj + (l - 1) * n, n, lw[l - 1], lh[l - 1], s);
     ADJ_CUDA(cudaMemcpy2DAsync(grad, sizeof(float) * pitch, d_glvl, sizeof(float) * lp[0], sizeof(float) * W,
                                (size_t)n * H, cudaMemcpyDeviceToDevice, s));
     if (gparams) ADJ_CUDA(cudaMemcpyAsync(gparams, d_gp, sizeof(double) * 4, cudaMemcpyDeviceToDevice, s));

@@ -2,7 +2,7 @@
 // inside namespace bimp_b200, after the forward kernels).
 //
 //   k_pyr_down_f        float pyramid level (pyrDown without uint8 rounding)
-//   k_pyr_down_f_adj    its transpose (scatter-add of the 5x5 taps)
+//   k_pyr_down_f_adj    its transpose
 //   k_stencil_bwd       gather form of d L / d C over the stencil window from
 //                       the ReLU states the forward stencil recorded (when
 //                       fftW == dataW, window column dataW is the torus
@@ -17,44 +17,120 @@
 //                       gives the window gradient, scattered to the level
 #pragma once
 
-__global__ void k_pyr_down_f(const PyrJobF* __restrict__ jobs) {
+__global__ void __launch_bounds__(256) k_pyr_down_f(const PyrJobF* __restrict__ jobs) {
   const PyrJobF j = jobs[blockIdx.z];
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
   if (x >= j.dw || y >= j.dh) return;
   const float w5[5] = {1.f, 4.f, 6.f, 4.f, 1.f};
-  int cols[5];
-#pragma unroll
-  for (int k = 0; k < 5; ++k) cols[k] = reflect101(2 * x + k - 2, j.sw);
   float acc = 0.f;
+  if (x >= 1 && 2 * x + 2 < j.sw && y >= 1 && 2 * y + 2 < j.sh) {
+    // inside: the five columns as two 8-byte loads and one (rows start
+    // 128-byte aligned), no reflection
+    const float* row = j.src + (size_t)(2 * y - 2) * j.sp + 2 * x - 2;
 #pragma unroll
-  for (int i = 0; i < 5; ++i) {
-    const float* row = j.src + (size_t)reflect101(2 * y + i - 2, j.sh) * j.sp;
-    float h = 0.f;
+    for (int i = 0; i < 5; ++i, row += j.sp) {
+      const float2 a = *reinterpret_cast<const float2*>(row), b = *reinterpret_cast<const float2*>(row + 2);
+      const float v[5] = {a.x, a.y, b.x, b.y, row[4]};
+      float h = 0.f;
 #pragma unroll
-    for (int k = 0; k < 5; ++k) h += w5[k] * row[cols[k]];
-    acc += w5[i] * h;
+      for (int k = 0; k < 5; ++k) h += w5[k] * v[k];
+      acc += w5[i] * h;
+    }
+  } else {
+    int cols[5];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) cols[k] = reflect101(2 * x + k - 2, j.sw);
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+      const float* row = j.src + (size_t)reflect101(2 * y + i - 2, j.sh) * j.sp;
+      float h = 0.f;
+#pragma unroll
+      for (int k = 0; k < 5; ++k) h += w5[k] * row[cols[k]];
+      acc += w5[i] * h;
+    }
   }
   j.dst[(size_t)y * j.dp + x] = acc * (1.0f / 256.0f);
 }
 
-// g_src(r101(2y+i), r101(2x+j)) += w_i w_j / 256 * g_dst(y, x)
-__global__ void k_pyr_down_f_adj(const PyrJobF* __restrict__ jobs) {
+// The transpose of the reflected, decimated window along one axis of n source
+// positions: weight w[k] with which source position p enters output Y0 + k (the
+// outputs past the ends get weight 0).  Position p itself, and next to a border
+// the window position -1, -2, n or n + 1 that reflects onto it, which lies in
+// the window of the same three outputs (n >= 5).
+__device__ __forceinline__ int pyr_adj_weights(int p, int n, float (&w)[3]) {
+  const int Y0 = (p - 1) >> 1, m = (n + 1) >> 1;
+  auto f = [](int d) { return d == 0 ? 6.f : d == 1 || d == -1 ? 4.f : d == 2 || d == -2 ? 1.f : 0.f; };
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const int Y = Y0 + k;
+    w[k] = f(p - 2 * Y);
+    if (p >= 1 && p <= 2) w[k] += f(-p - 2 * Y);
+    if (p >= n - 3 && p <= n - 2) w[k] += f(2 * n - 2 - p - 2 * Y);
+    if (Y < 0 || Y >= m) w[k] = 0.f;
+  }
+  return Y0;
+}
+
+// g_src(r101(2y+i), r101(2x+j)) += w_i w_j / 256 * g_dst(y, x), gathered: a
+// thread adds what reaches four adjacent pixels of the finer level, inside from
+// 3 x 4 outputs (columns, then rows).  (The adjoint takes sides of 16 and more,
+// so levels of fewer than 5 rows or columns come from coarse scales only: those
+// go output by output.)  Scattering 25 atomics per output took 55 + 19 us for
+// the two steps of 16 x 512 x 512 (six scales), this 24 + 13.
+__global__ void __launch_bounds__(256) k_pyr_down_f_adj(const PyrJobF* __restrict__ jobs) {
   const PyrJobF j = jobs[blockIdx.z];
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  const int x = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
-  if (x >= j.dw || y >= j.dh) return;
-  const float g = j.src[(size_t)y * j.sp + x] * (1.0f / 256.0f);   // here src = level l gradient
-  if (g == 0.f) return;
+  if (x >= j.sw || y >= j.sh) return;
+  float* __restrict__ dst = j.dst + (size_t)y * j.dp + x;
+  if (j.sw >= 5 && j.sh >= 5) {
+    float wy[3];
+    const int Y0 = pyr_adj_weights(y, j.sh, wy);
+    if (x >= 4 && x + 8 < j.sw) {   // no border in x
+      float4 d = *reinterpret_cast<const float4*>(dst);
+      const float* src = j.src + (x >> 1) - 1;
+      float v[4] = {0.f, 0.f, 0.f, 0.f};   // columns x/2 - 1 .. x/2 + 2
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        if (wy[i] == 0.f) continue;
+        const float* row = src + (size_t)(Y0 + i) * j.sp;
+        const float2 m = __ldg(reinterpret_cast<const float2*>(row + 1));   // x/2 is even
+        const float c[4] = {__ldg(row), m.x, m.y, __ldg(row + 3)};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] = fmaf(wy[i], c[k], v[k]);
+      }
+      constexpr float s1 = 1.f / 256.f, s4 = 4.f / 256.f, s6 = 6.f / 256.f;
+      d.x += s1 * (v[0] + v[2]) + s6 * v[1];
+      d.y += s4 * (v[1] + v[2]);
+      d.z += s1 * (v[1] + v[3]) + s6 * v[2];
+      d.w += s4 * (v[2] + v[3]);
+      *reinterpret_cast<float4*>(dst) = d;
+      return;
+    }
+    for (int e = 0; e < 4 && x + e < j.sw; ++e) {
+      float wx[3], acc = 0.f;
+      const int X0 = pyr_adj_weights(x + e, j.sw, wx);
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+          if (wy[i] != 0.f && wx[k] != 0.f)
+            acc = fmaf(wy[i] * wx[k], __ldg(j.src + (size_t)(Y0 + i) * j.sp + X0 + k), acc);
+      dst[e] += acc * (1.0f / 256.0f);
+    }
+    return;
+  }
   const float w5[5] = {1.f, 4.f, 6.f, 4.f, 1.f};
-  int cols[5];
-#pragma unroll
-  for (int k = 0; k < 5; ++k) cols[k] = reflect101(2 * x + k - 2, j.sw);
-#pragma unroll
-  for (int i = 0; i < 5; ++i) {
-    float* row = j.dst + (size_t)reflect101(2 * y + i - 2, j.sh) * j.dp;
-#pragma unroll
-    for (int k = 0; k < 5; ++k) atomicAdd(row + cols[k], w5[i] * w5[k] * g);
+  for (int e = 0; e < 4 && x + e < j.sw; ++e) {
+    float acc = 0.f;
+    for (int Y = 0; Y < j.dh; ++Y)
+      for (int i = 0; i < 5; ++i)
+        if (reflect101(2 * Y + i - 2, j.sh) == y)
+          for (int X = 0; X < j.dw; ++X)
+            for (int k = 0; k < 5; ++k)
+              if (reflect101(2 * X + k - 2, j.sw) == x + e) acc += w5[i] * w5[k] * j.src[(size_t)Y * j.sp + X];
+    dst[e] += acc * (1.0f / 256.0f);
   }
 }
 
@@ -83,10 +159,76 @@ constexpr int kStBwThreads = 256;
 // at q (ScaleDev::bits).  Sources lie within +-8 of p.  The tangential and
 // radial weights are constants here; their own gradients come from
 // the forward stencil.
+//
+// A source's weight and states sit side by side in shared memory (one 8-byte
+// load), and with a built-in offset set every address is an immediate off the
+// pixel's and sources that several orientations share are loaded once (33
+// instead of 80 loads a pixel; the run-time offsets cost 48 more): 238 -> 190 us
+// for 16 x 512 x 512, 6 scales. What is left is those loads (80% of the L1 rate:
+// two wavefronts each) and the selections (72% of the issue slots);
+// multiply-adds under a predicate instead of selections: 210 us.
+template <int PAT>
+__device__ __forceinline__ void stencil_bwd_rows(const uint2* __restrict__ sQ, const int (*sOff)[6],
+                                                 const ScaleDev* __restrict__ sd, int x0, int y0) {
+  constexpr int sets[kNumOffsetSets][6][8] = BIMP_OFFSET_SETS;
+  const int t = threadIdx.x, W = sd->dataW, H = sd->dataH, lx = t & 31, px = x0 + lx;
+  const float wT = sd->wTan, wR = sd->wRad, gR = sd->radialGain * wR;
+  const int wrapW = sd->wrapW, cPitch = sd->cPitch;
+  const long long cStride = sd->cStride;
+  float* __restrict__ gC = sd->gC;
+#pragma unroll 1
+  for (int ly = t >> 5; ly < kStY; ly += kStBwThreads / 32) {
+    const int py = y0 + ly;
+    if (py > H + 1 || px > W) continue;           // row H + 1: read by no stencil, gathers 0
+    const uint2* q0 = sQ + (ly + kHalo) * kBwQW + lx + kHalo;   // p in source-pixel coordinates
+    auto at = [&](int dy, int dx) { return q0[dy * kBwQW + dx]; };
+    // the source's weight where its states have the bit
+    auto weight = [](uint2 q, unsigned int bit) { return q.y & bit ? __uint_as_float(q.x) : 0.f; };
+    const uint2 c = at(0, 0);
+    const float m0 = __uint_as_float(c.x), mR = wR * m0;
+    float g[kNumOri];
+#pragma unroll
+    for (int o = 0; o < kNumOri; ++o) {
+      const int op = (o + kNumOri / 2) % kNumOri;
+      auto off = [&](int k, int oo) {
+        if constexpr (PAT > 0) return sets[PAT - 1][k][oo];
+        else return sOff[oo][k];
+      };
+      const int o1 = off(0, o), o2 = off(1, o), i1 = off(2, o), i2 = off(3, o);
+      const int ph1 = off(4, op), ph2 = off(5, op);
+      const unsigned int bd = 1u << (4 * o), bt = 2u << (4 * o), br = 4u << (4 * o), br1 = 8u << (4 * o);
+      const unsigned int pr = 4u << (4 * op), pr1 = 8u << (4 * op);
+      // double-stopped: p is the centre of q = p, and a -1/2 tap of q = p +- 2 offset
+      float v = weight(c, bd);
+      v = fmaf(-0.5f, weight(at(2 * o1, -2 * o2), bd), v);
+      v = fmaf(-0.5f, weight(at(-2 * o1, 2 * o2), bd), v);
+      // tangential: p is read by q = p + i (as C(q - i)) and by q = p (centre)
+      v = fmaf(-wT, weight(at(i1, i2), bt), v);
+      v = fmaf(wT, weight(c, bt), v);
+      // radial, o as the centre orientation (both terms when r1 > 0)
+      v -= c.y & br ? mR * (c.y & br1 ? 2.f : 1.f) : 0.f;
+      // radial, o as the perpendicular map of op: read at q + h (r1) and q - h (r)
+      const uint2 q1 = at(-ph1, -ph2);
+      v = fmaf(gR, q1.y & pr ? weight(q1, pr1) : 0.f, v);
+      v = fmaf(gR, weight(at(ph1, ph2), pr), v);
+      g[o] = v;
+    }
+    // fftW == dataW: window column dataW of row r is the torus element
+    // (r + 1, 0); its gradient goes to gWrap[o][r], which the tile
+    // backward adds at (r + 1, 0)
+    const bool wrapped = wrapW && px == W;
+    float* dst = gC + (size_t)py * cPitch + px;
+#pragma unroll
+    for (int o = 0; o < kNumOri; ++o) {
+      if (wrapped && py <= H) sd->gWrap[o * (H + 1) + py] = g[o];
+      dst[o * cStride] = wrapped ? 0.f : g[o];
+    }
+  }
+}
+
 __global__ void __launch_bounds__(kStBwThreads)
 k_stencil_bwd(const ScaleDev* __restrict__ sds, const int2* __restrict__ work) {
-  __shared__ float sM[kBwQW * kBwQW];
-  __shared__ unsigned int sBits[kBwQW * kBwQW];
+  __shared__ uint2 sQ[kBwQW * kBwQW];   // per source pixel: loss weight, ReLU states (0 outside the map)
   __shared__ int sOff[kNumOri][6];
   const int2 item = work[blockIdx.x];
   const ScaleDev* __restrict__ sd = sds + item.x;
@@ -95,74 +237,29 @@ k_stencil_bwd(const ScaleDev* __restrict__ sds, const int2* __restrict__ work) {
   const int by = item.y / nbx, bx = item.y - by * nbx;
   const int x0 = bx * kStX, y0 = by * kStY;
   const int t = threadIdx.x;
-  const float gain = sd->radialGain, wT = sd->wTan, wR = sd->wRad;
-  const int wrapW = sd->wrapW;
   if (t < kNumOri) {
     sOff[t][0] = sd->es1[t]; sOff[t][1] = sd->es2[t];
     sOff[t][2] = sd->in1[t]; sOff[t][3] = sd->in2[t];
     sOff[t][4] = sd->ih1[t]; sOff[t][5] = sd->ih2[t];
   }
   const int dp = sd->dPitch;
-  for (int idx = t; idx < kBwQW * kBwQW; idx += kStBwThreads) {
+  const float* __restrict__ M = sd->M;
+  const unsigned int* __restrict__ bits = sd->bits;
+#pragma unroll
+  for (int i = 0; i < kBwQW * kBwQW / kStBwThreads; ++i) {
+    const int idx = t + kStBwThreads * i;
     const int ly = idx / kBwQW, lx = idx - ly * kBwQW;
     const int gy = y0 - kHalo + ly, gx = x0 - kHalo + lx;
     const bool in = gy >= 0 && gy < H && gx >= 0 && gx < W;
-    sM[idx] = in ? sd->M[(size_t)gy * W + gx] : 0.f;
-    sBits[idx] = in ? sd->bits[(size_t)gy * dp + gx] : 0u;
+    sQ[idx] = in ? make_uint2(__float_as_uint(__ldg(M + (size_t)gy * W + gx)), __ldg(bits + (size_t)gy * dp + gx))
+                 : make_uint2(0u, 0u);
   }
   __syncthreads();
-  float* __restrict__ gC = sd->gC;
-  const int cPitch = sd->cPitch;
-  const long long cStride = sd->cStride;
-  const int lx = t & 31;
-  for (int ly = t >> 5; ly < kStY; ly += kStBwThreads / 32) {
-    const int py = y0 + ly, px = x0 + lx;
-    if (py > H + 1 || px > W) continue;           // row H + 1: read by no stencil, gathers 0
-    const int qy = ly + kHalo, qx = lx + kHalo;   // p in source-pixel coordinates
-    auto at = [&](int dy, int dx) { return (qy + dy) * kBwQW + (qx + dx); };
-    const unsigned int b0 = sBits[at(0, 0)];
-    const float m0 = sM[at(0, 0)];
-#pragma unroll
-    for (int o = 0; o < kNumOri; ++o) {
-      const int op = (o + kNumOri / 2) % kNumOri;
-      const int o1 = sOff[o][0], o2 = sOff[o][1], i1 = sOff[o][2], i2 = sOff[o][3];
-      const int ph1 = sOff[op][4], ph2 = sOff[op][5];
-      const unsigned int bd = 1u << (4 * o), bt = 2u << (4 * o), br = 4u << (4 * o), br1 = 8u << (4 * o);
-      const unsigned int pr = 4u << (4 * op), pr1 = 8u << (4 * op);
-      float g = 0.f;
-      // double-stopped: p is the centre of q = p, and a -1/2 tap of q = p +- 2 offset
-      if (b0 & bd) g += m0;
-      {
-        const int ka = at(2 * o1, -2 * o2), kb = at(-2 * o1, 2 * o2);
-        if (sBits[ka] & bd) g -= 0.5f * sM[ka];
-        if (sBits[kb] & bd) g -= 0.5f * sM[kb];
-      }
-      // tangential: p is read by q = p + i (as C(q - i)) and by q = p (centre)
-      {
-        const int kq = at(i1, i2);
-        if (sBits[kq] & bt) g -= wT * sM[kq];
-        if (b0 & bt) g += wT * m0;
-      }
-      // radial, o as the centre orientation (both terms when r1 > 0)
-      if (b0 & br) g -= wR * m0 * ((b0 & br1) ? 2.f : 1.f);
-      // radial, o as the perpendicular map of op: read at q + h (r1) and q - h (r)
-      {
-        const int k1 = at(-ph1, -ph2), k2 = at(ph1, ph2);
-        const unsigned int b1 = sBits[k1], b2 = sBits[k2];
-        if ((b1 & pr) && (b1 & pr1)) g += gain * wR * sM[k1];
-        if (b2 & pr) g += gain * wR * sM[k2];
-      }
-      // fftW == dataW: window column dataW of row r is the torus element
-      // (r + 1, 0); its gradient goes to gWrap[o][r], which the tile
-      // backward adds at (r + 1, 0)
-      if (wrapW && px == W) {
-        if (py <= H) sd->gWrap[o * (H + 1) + py] = g;
-        g = 0.f;
-      }
-      gC[(size_t)o * cStride + (size_t)py * cPitch + px] = g;
-    }
-  }
+  if (sd->pattern == 1) stencil_bwd_rows<1>(sQ, sOff, sd, x0, y0);
+  else if (sd->pattern == 2) stencil_bwd_rows<2>(sQ, sOff, sd, x0, y0);
+  else stencil_bwd_rows<0>(sQ, sOff, sd, x0, y0);
 }
+static_assert(kBwQW * kBwQW % kStBwThreads == 0, "staging loop");
 
 // --- tile backward -----------------------------------------------------------
 // |e + i o| at or below kMagFloor counts as zero: no gradient flows through

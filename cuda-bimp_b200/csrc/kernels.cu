@@ -1382,7 +1382,7 @@ void launch_pyr_f(const PyrJobF* d_jobs, int njobs, int maxW, int maxH, cudaStre
   k_pyr_down_f<<<g, b, 0, s>>>(d_jobs);
 }
 void launch_pyr_f_adj(const PyrJobF* d_jobs, int njobs, int maxW, int maxH, cudaStream_t s) {
-  dim3 b(32, 8), g((maxW + 31) / 32, (maxH + 7) / 8, njobs);
+  dim3 b(32, 8), g((maxW + 127) / 128, (maxH + 7) / 8, njobs);
   k_pyr_down_f_adj<<<g, b, 0, s>>>(d_jobs);
 }
 void launch_stencil_bwd(const ScaleDev* d_sd, const int2* d_work, int nwork, cudaStream_t s) {
