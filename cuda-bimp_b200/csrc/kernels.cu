@@ -60,12 +60,12 @@ __device__ __forceinline__ int reflect101(int i, int n) {
 constexpr int pyr_tile(int K) { return 32 >> (K - 1); }
 
 constexpr int pyr_side(int K, int m) { return m == K ? pyr_tile(K) : 2 * pyr_side(K, m + 1) + 3; }
-// Shared memory of the computed levels 1..K (square regions).
-constexpr int pyr_smem(int K) {
-  return K == 3 ? pyr_side(3, 1) * pyr_side(3, 1) + pyr_side(3, 2) * pyr_side(3, 2) + pyr_side(3, 3) * pyr_side(3, 3)
-       : K == 2 ? pyr_side(2, 1) * pyr_side(2, 1) + pyr_side(2, 2) * pyr_side(2, 2)
-                : pyr_side(1, 1) * pyr_side(1, 1);
-}
+// Rows of a computed level's region and of the horizontal sums start 4-byte
+// aligned (an even side has one spare column at least where it is odd).
+constexpr int pyr_pitch(int K, int m) { return (pyr_side(K, m) + 3) & ~3; }
+// First byte of level m's region (m >= 1) in the shared memory of the computed
+// levels; pyr_off(K, K + 1) is its size.
+constexpr int pyr_off(int K, int m) { return m <= 1 ? 0 : pyr_off(K, m - 1) + pyr_side(K, m - 1) * pyr_pitch(K, m - 1); }
 // The source region is staged as 16-byte chunks: the chunks of a region row
 // cover its S0 bytes after a lead of up to 15 bytes (the region's first
 // column rounded down to a 16-byte boundary).
@@ -74,9 +74,7 @@ constexpr int kPyrThreads = 256;
 
 // Largest horizontal-pass buffer of a K-level launch (rows of the level
 // above x columns of the level computed).
-constexpr int pyr_hbuf(int K) {
-  return K == 3 ? pyr_side(3, 0) * pyr_side(3, 1) : K == 2 ? pyr_side(2, 0) * pyr_side(2, 1) : pyr_side(1, 0) * pyr_side(1, 1);
-}
+constexpr int pyr_hbuf(int K) { return (pyr_side(K, 0) + 2) * pyr_pitch(K, 1); }   // + 2 rows read by the last row pair
 
 // Level M of a K-level launch from level M - 1: regions of side
 // pyr_side(K, M - 1) (in) and pyr_side(K, M) (out) in shared memory.  A
@@ -87,19 +85,27 @@ constexpr int pyr_hbuf(int K) {
 // copies do not overlap.  Then every region runs the same two passes:
 // output column c takes input columns 2 c .. 2 c + 4, output row r rows
 // 2 r .. 2 r + 4 (exact integer sums: the same values as reflecting each
-// tap), two outputs per item.
+// tap).
+//
+// Integer arithmetic bounds it, so both passes work on packed values: the
+// horizontal one takes four taps of a byte sum in one dp4a (two outputs an
+// item from two or three words), the vertical one two columns' 16-bit sums in
+// one register (two rows an item; the largest sum with its rounding, 255 * 256
+// + 128, fits 16 bits).  With the launch behind it overlapped, a 4K pyramid
+// takes 31 us and a 1080p one 11.5 (39 and 12.4 byte by byte, the launches in
+// series); below that size the two launches' latency is the whole time.
 template <int K, int M>
-__device__ __forceinline__ void pyr_level(const PyrJob& j, const int (&loY)[K + 1], const int (&loX)[K + 1],
-                                          const int (&off)[K + 1], int oy, int ox, int lead, uint8_t* s_raw,
-                                          uint8_t* s_lvl, uint16_t* s_h, int t) {
+__device__ __forceinline__ void pyr_level(const PyrJob& j, const int (&loY)[K + 1], const int (&loX)[K + 1], int oy,
+                                          int ox, int lead, uint8_t* s_raw, uint8_t* s_lvl, uint16_t* s_h, int t) {
   constexpr int Si = pyr_side(K, M - 1), So = pyr_side(K, M), Sp = (So + 1) / 2;
-  constexpr int ip = M == 1 ? 16 * pyr_chunks(K) : Si;   // row pitch of the level above in shared memory
+  constexpr int ip = M == 1 ? 16 * pyr_chunks(K) : pyr_pitch(K, M - 1);   // row pitch of the level above
+  constexpr int hp = pyr_pitch(K, M), op = pyr_pitch(K, M);
   constexpr int own = pyr_tile(K) << (K - M);
   const int Wi = M == 1 ? j.sw : j.dw[M - 2], Hi = M == 1 ? j.sh : j.dh[M - 2];
   const int Wo = j.dw[M - 1], Ho = j.dh[M - 1];
   const int ownY = oy << (K - M), ownX = ox << (K - M);
-  uint8_t* in = M == 1 ? s_raw + lead : s_lvl + off[M - 1];
-  uint8_t* outS = s_lvl + off[M];
+  uint8_t* in = M == 1 ? s_raw + lead : s_lvl + pyr_off(K, M - 1);
+  uint8_t* outS = s_lvl + pyr_off(K, M);
   uint8_t* dst = j.dst[M - 1];
   const int dp = j.dp[M - 1];
   const int ly = loY[M - 1], lx = loX[M - 1];
@@ -127,37 +133,50 @@ __device__ __forceinline__ void pyr_level(const PyrJob& j, const int (&loY)[K + 
     }
     __syncthreads();
   }
-  // horizontal pass: columns c, c + 1 share input columns 2 c + 2 .. 2 c + 4
-  // (for an odd So the last item's second output is not stored; its two
-  // extra input bytes lie inside the buffers)
+  // horizontal pass: columns c, c + 1 (c even) of row r from bytes a0 .. a6 at
+  // input column 2 c.  A computed level's rows are 4-byte aligned; the staged
+  // source's lead is 2 mod 4 (regions start at 2 (2 x - ..) - 2).
+  constexpr unsigned kW = 0x04060401u;   // weights 1, 4, 6, 4
   for (int idx = t; idx < Si * Sp; idx += kPyrThreads) {
     const int r = idx / Sp, c = 2 * (idx - r * Sp);
-    const uint8_t* a = in + r * ip + 2 * c;
-    const int a0 = a[0], a1 = a[1], a2 = a[2], a3 = a[3], a4 = a[4], a5 = a[5], a6 = a[6];
-    s_h[r * So + c] = (uint16_t)(a0 + 4 * a1 + 6 * a2 + 4 * a3 + a4);
-    if (c + 1 < So) s_h[r * So + c + 1] = (uint16_t)(a2 + 4 * a3 + 6 * a4 + 4 * a5 + a6);
+    unsigned lo, hi;
+    if constexpr (M == 1) {
+      const unsigned* w = reinterpret_cast<const unsigned*>(in + r * ip + 2 * c - 2);
+      const unsigned w0 = w[0], w1 = w[1], w2 = w[2];   // a-2 a-1 a0 a1 | a2 .. a5 | a6 ..
+      lo = __dp4a(__byte_perm(w0, w1, 0x5432), kW, (w1 >> 16) & 255u);
+      hi = __dp4a(w1, kW, w2 & 255u);
+    } else {
+      const unsigned* w = reinterpret_cast<const unsigned*>(in + r * ip + 2 * c);
+      const unsigned w0 = w[0], w1 = w[1];   // a0 .. a3 | a4 .. a7
+      lo = __dp4a(w0, kW, w1 & 255u);
+      hi = __dp4a(__byte_perm(w0, w1, 0x5432), kW, (w1 >> 16) & 255u);
+    }
+    *reinterpret_cast<unsigned*>(s_h + r * hp + c) = lo | hi << 16;
   }
   __syncthreads();
   // vertical pass: rows r, r + 1 share h-pass rows 2 r + 2 .. 2 r + 4;
   // rounding to nearest with ties to even; the owned outputs inside the
   // level go to the level buffer
-  for (int idx = t; idx < Sp * So; idx += kPyrThreads) {
-    const int rp = idx / So, c = idx - rp * So, r = 2 * rp;
-    const uint16_t* a = s_h + 2 * r * So + c;
-    const int b0 = a[0], b1 = a[So], b2 = a[2 * So], b3 = a[3 * So], b4 = a[4 * So], b5 = a[5 * So],
-              b6 = a[6 * So];
+  for (int idx = t; idx < Sp * Sp; idx += kPyrThreads) {
+    const int rp = idx / Sp, c = 2 * (idx - rp * Sp), r = 2 * rp;
+    const unsigned* a = reinterpret_cast<const unsigned*>(s_h + 2 * r * hp + c);
+    const unsigned b0 = a[0], b1 = a[hp / 2], b2 = a[hp], b3 = a[3 * hp / 2], b4 = a[2 * hp], b5 = a[5 * hp / 2],
+                   b6 = a[3 * hp];
     const int x = loX[M] + c;
-    const bool xin = x >= ownX && x < ownX + own && x < Wo;
+    const bool xin = x >= ownX && x < ownX + own && x < Wo;   // x and ownX are even
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       if (h == 1 && r + 1 >= So) break;
-      const int acc = h ? b2 + 4 * b3 + 6 * b4 + 4 * b5 + b6 : b0 + 4 * b1 + 6 * b2 + 4 * b3 + b4;
-      const int q = acc >> 8;
-      int v = (acc + 127 + (q & 1)) >> 8;
-      v = v > 255 ? 255 : v;
-      outS[(r + h) * So + c] = (uint8_t)v;
+      const unsigned acc = h ? b2 + b6 + 4 * (b3 + b5) + 6 * b4 : b0 + b4 + 4 * (b1 + b3) + 6 * b2;
+      const unsigned v = ((acc + 0x007f007fu + ((acc >> 8) & 0x00010001u)) >> 8) & 0x00ff00ffu;
+      const uint16_t two = (uint16_t)(v | v >> 8);
+      *reinterpret_cast<uint16_t*>(outS + (r + h) * op + c) = two;
       const int y = loY[M] + r + h;
-      if (xin && y >= ownY && y < ownY + own && y < Ho) dst[(size_t)y * dp + x] = (uint8_t)v;
+      if (xin && y >= ownY && y < ownY + own && y < Ho) {
+        uint8_t* q = dst + (size_t)y * dp + x;
+        if (x + 1 < Wo) *reinterpret_cast<uint16_t*>(q) = two;
+        else *q = (uint8_t)two;
+      }
     }
   }
   __syncthreads();
@@ -167,9 +186,9 @@ template <int K>
 __global__ void __launch_bounds__(kPyrThreads) k_pyr_down(const PyrJob* __restrict__ jobs,
                                                            unsigned int* __restrict__ reset, int resetWords) {
   constexpr int S0 = pyr_side(K, 0), CPR = pyr_chunks(K), SP = 16 * CPR;
-  __shared__ __align__(16) uint8_t s_raw[S0 * SP];   // source region, row pitch SP
-  __shared__ uint8_t s_lvl[pyr_smem(K)];             // levels 1..K
-  __shared__ uint16_t s_h[pyr_hbuf(K) + 2 * pyr_side(K, 1)];   // + 2 rows read by the last row pair
+  __shared__ __align__(16) uint8_t s_raw[S0 * SP + 16];   // source region, row pitch SP (+ a word read past it)
+  __shared__ __align__(16) uint8_t s_lvl[pyr_off(K, K + 1) + 4];   // levels 1..K (+ a word read past the last row)
+  __shared__ __align__(16) uint16_t s_h[pyr_hbuf(K)];
   griddep_launch_dependents();
   // the detection's reset (the map maxima and the fault word), done here
   // instead of by a memset of its own: every later kernel waits for this grid
@@ -180,7 +199,8 @@ __global__ void __launch_bounds__(kPyrThreads) k_pyr_down(const PyrJob* __restri
   constexpr int T = pyr_tile(K);
   const int oy = blockIdx.y * T, ox = blockIdx.x * T;
   if (oy >= j.dh[K - 1] || ox >= j.dw[K - 1]) return;
-  int loY[K + 1], loX[K + 1], off[K + 1];
+  if (!reset) griddep_wait();   // a later launch of the chain: the level above comes from the previous kernel
+  int loY[K + 1], loX[K + 1];
   loY[K] = oy;
   loX[K] = ox;
 #pragma unroll
@@ -188,10 +208,6 @@ __global__ void __launch_bounds__(kPyrThreads) k_pyr_down(const PyrJob* __restri
     loY[m - 1] = 2 * loY[m] - 2;
     loX[m - 1] = 2 * loX[m] - 2;
   }
-  off[0] = 0;
-  off[1] = 0;
-#pragma unroll
-  for (int m = 2; m <= K; ++m) off[m] = off[m - 1] + pyr_side(K, m - 1) * pyr_side(K, m - 1);
   const int t = threadIdx.x;
   // Source region as 16-byte chunks (level rows start 16-byte aligned and
   // their pitch is a multiple of 16, so a chunk that starts inside the pitch
@@ -219,9 +235,9 @@ __global__ void __launch_bounds__(kPyrThreads) k_pyr_down(const PyrJob* __restri
     }
   }
   __syncthreads();
-  pyr_level<K, 1>(j, loY, loX, off, oy, ox, lead, s_raw, s_lvl, s_h, t);
-  if constexpr (K >= 2) pyr_level<K, 2>(j, loY, loX, off, oy, ox, lead, s_raw, s_lvl, s_h, t);
-  if constexpr (K >= 3) pyr_level<K, 3>(j, loY, loX, off, oy, ox, lead, s_raw, s_lvl, s_h, t);
+  pyr_level<K, 1>(j, loY, loX, oy, ox, lead, s_raw, s_lvl, s_h, t);
+  if constexpr (K >= 2) pyr_level<K, 2>(j, loY, loX, oy, ox, lead, s_raw, s_lvl, s_h, t);
+  if constexpr (K >= 3) pyr_level<K, 3>(j, loY, loX, oy, ox, lead, s_raw, s_lvl, s_h, t);
 }
 
 // ---------------------------------------------------------------------------
@@ -1347,9 +1363,9 @@ void launch_pyr(const PyrJob* d_jobs, int njobs, int levels, int maxW, int maxH,
   if (njobs <= 0 || levels <= 0) return;
   const int T = 32 >> (levels - 1);
   dim3 g((maxW + T - 1) / T, (maxH + T - 1) / T, njobs);
-  if (levels == 3) k_pyr_down<3><<<g, kPyrThreads, 0, s>>>(d_jobs, reset, resetWords);
-  else if (levels == 2) k_pyr_down<2><<<g, kPyrThreads, 0, s>>>(d_jobs, reset, resetWords);
-  else k_pyr_down<1><<<g, kPyrThreads, 0, s>>>(d_jobs, reset, resetWords);
+  auto k = levels == 3 ? k_pyr_down<3> : levels == 2 ? k_pyr_down<2> : k_pyr_down<1>;
+  // the launches after the first (the one with the reset) wait in the kernel
+  launch_ex(k, g, kPyrThreads, 0, s, !reset, d_jobs, reset, resetWords);
 }
 void launch_gabor(const ScaleDev* d_sd, const TileWork* d_work, int nwork, int grid, unsigned int* d_fault,
                   cudaStream_t s, bool pipelined, bool pdl) {
