@@ -69,6 +69,8 @@ struct bimp_adjoint {
   std::vector<ScaleHost> geo;
   char* mem = nullptr;
   size_t bytes = 0;
+  char* keep = nullptr;                   // the forward's responses and tile spectra for the backward, or null
+  size_t keepBytes = 0;
   std::vector<ScaleDev> h_sd;
   ScaleDev* d_sd = nullptr;
   // The tile kernels' work plans, one per chunk of images: the balanced split
@@ -104,6 +106,32 @@ struct bimp_adjoint {
   double* d_loss = nullptr;               // [0] loss, [1..4] parameter gradients
   double* d_gp = nullptr;
   unsigned int* d_max = nullptr;          // per entry + fault word
+
+  // Memory for the forward's e + i o and tile spectra, which let the backward
+  // start from them instead of transforming every tile again.  It is taken
+  // where the program has plenty: up to kKeepBudget and an eighth of the
+  // device's free memory (BIMP_ADJOINT_KEEP=0: none, for tests); otherwise, or
+  // if it cannot be had, the backward recomputes both.
+  void reserve_kept(const std::vector<ScaleDev>& sds, std::vector<size_t>& offZ, std::vector<size_t>& offX) {
+    size_t at = 0;
+    for (const ScaleDev& d : sds) {
+      offZ.push_back(at);
+      at += up(sizeof(float2) * kKeptBlock * (size_t)kNumOri * d.tilesX * kept_column_blocks(d), 256);
+      offX.push_back(at);
+      at += up(sizeof(float2) * kSpecHalf * (size_t)d.tilesX * d.tilesY, 256);
+    }
+    constexpr size_t kKeepBudget = size_t(8) << 30;
+    size_t freeB = 0, totalB = 0;
+    const char* k = std::getenv("BIMP_ADJOINT_KEEP");
+    if ((k && std::atoi(k) == 0) || cudaMemGetInfo(&freeB, &totalB) != cudaSuccess) return;
+    if (at > kKeepBudget || at > freeB / 8) return;
+    if (cudaMalloc(&keep, at) != cudaSuccess) {
+      cudaGetLastError();
+      keep = nullptr;
+      return;
+    }
+    keepBytes = at;
+  }
 
   int build(int dev, int w, int h, int ni, const float* lambdas, int nl, const bimp_params& p) {
     device = dev;
@@ -245,6 +273,12 @@ struct bimp_adjoint {
     nTiles = static_cast<int>(tiles.size());
     nSten = static_cast<int>(sten.size());
     nStenB = static_cast<int>(stenB.size());
+    // the kernel that pipelines the forward (BIMP_TILE_KERNEL=pipelined) keeps nothing
+    const char* kern = std::getenv("BIMP_TILE_KERNEL");
+    pipelined = kern && std::strcmp(kern, "pipelined") == 0;
+    for (const ScaleDev& d : sds) pipelined = pipelined && d.V <= pipelined_tile_max_valid();
+    std::vector<size_t> offZ, offX;   // per entry, in `keep`
+    if (!pipelined) reserve_kept(sds, offZ, offX);
     std::vector<TileWork> plans;
     for (int i0 = 0; i0 < n; i0 += chunk) {
       const std::vector<TileWork> part(tiles.begin() + tileStart[i0], tiles.begin() + tileStart[std::min(n, i0 + chunk)]);
@@ -258,7 +292,7 @@ struct bimp_adjoint {
         return p.grid;
       };
       add(fwdPlan, kForwardCost);
-      bwdGrid = std::max(bwdGrid, add(bwdPlan, kBackwardCost));
+      bwdGrid = std::max(bwdGrid, add(bwdPlan, keep ? kBackwardKeptCost : kBackwardCost));
     }
     const size_t offSd = take(sizeof(ScaleDev) * sds.size());
     const size_t offT2 = take(sizeof(TileWork) * plans.size());
@@ -272,6 +306,13 @@ struct bimp_adjoint {
     const size_t offMaps = take(kTensorMapBytes * sds.size());
     bytes = at;
     cudaError_t e = cudaMalloc(&mem, bytes);
+    if (e != cudaSuccess && keep) {   // what the adjoint cannot do without comes first
+      cudaGetLastError();
+      cudaFree(keep);
+      keep = nullptr;
+      keepBytes = 0;
+      e = cudaMalloc(&mem, bytes);
+    }
     if (e != cudaSuccess) {
       mem = nullptr;
       return afail(BIMP_ERR_NOMEM, "cudaMalloc of " + std::to_string(bytes) + " bytes failed");
@@ -301,7 +342,8 @@ struct bimp_adjoint {
       d.bwB = dBB + (size_t)si * kNumOri * kSpecHalf;
       const size_t slot = (size_t)(i % chunk) * nScales + si;   // chunk scratch shared across chunks
       d.C = reinterpret_cast<float*>(b + offC[slot]);
-      d.Z = nullptr;
+      d.Z = keep ? reinterpret_cast<float2*>(keep + offZ[e2]) : nullptr;
+      d.X = keep ? reinterpret_cast<float2*>(keep + offX[e2]) : nullptr;
       d.gC = reinterpret_cast<float*>(b + offGC[slot]);
       d.gWrap = reinterpret_cast<float*>(b + offGW[slot]);
       d.D = reinterpret_cast<float*>(b + offD[e2]);
@@ -317,10 +359,6 @@ struct bimp_adjoint {
       for (size_t e2 = 0; e2 < sds.size(); ++e2) sds[e2].cMap = b + offMaps + e2 * kTensorMapBytes;
     }
     h_sd = sds;
-    // the phased forward tile kernel unless BIMP_TILE_KERNEL=pipelined
-    const char* kern = std::getenv("BIMP_TILE_KERNEL");
-    pipelined = kern && std::strcmp(kern, "pipelined") == 0;
-    for (const ScaleDev& d : sds) pipelined = pipelined && d.V <= pipelined_tile_max_valid();
     d_sd = reinterpret_cast<ScaleDev*>(b + offSd);
     d_tiles = reinterpret_cast<TileWork*>(b + offT2);
     d_sten = reinterpret_cast<int2*>(b + offSt);
@@ -376,7 +414,7 @@ struct bimp_adjoint {
     for (int i0 = 0; i0 < n; i0 += chunk) {
       const int i1 = std::min(n, i0 + chunk);
       const Plan& p = fwdPlan[i0 / chunk];
-      launch_gabor_flt(d_sd, d_tiles + p.first, p.items, p.grid, fault, s, pipelined);
+      launch_gabor_flt(d_sd, d_tiles + p.first, p.items, p.grid, fault, s, pipelined, keep != nullptr);
       launch_stencil(d_sd, d_sten + stenStart[i0], stenStart[i1] - stenStart[i0], fault, s, kStencilAdj, false, d_loss,
                      d_gp);
     }
@@ -394,7 +432,7 @@ struct bimp_adjoint {
       const int i1 = std::min(n, i0 + chunk);
       launch_stencil_bwd(d_sd, d_stenB + stenBStart[i0], stenBStart[i1] - stenBStart[i0], s);
       const Plan& p = bwdPlan[i0 / chunk];
-      launch_gabor_bwd(d_sd, d_tiles + p.first, p.items, p.grid, d_xscr, d_gp, s);
+      launch_gabor_bwd(d_sd, d_tiles + p.first, p.items, p.grid, d_xscr, d_gp, s, keep != nullptr);
     }
     for (int l = maxLevel; l >= 1; --l) launch_pyr_f_adj(d_pyrAdj + (l - 1) * n, n, lw[l - 1], lh[l - 1], s);
     ADJ_CUDA(cudaMemcpy2DAsync(grad, sizeof(float) * pitch, d_glvl, sizeof(float) * lp[0], sizeof(float) * W,
@@ -425,6 +463,7 @@ int bimp_adjoint_create(bimp_adjoint** out, int width, int height, int n_images,
   rc = a->build(dev, width, height, n_images, lambdas, n_lambdas, p);
   if (rc != BIMP_OK) {
     if (a->mem) cudaFree(a->mem);
+    if (a->keep) cudaFree(a->keep);
     delete a;
     return rc;
   }
@@ -436,13 +475,14 @@ int bimp_adjoint_destroy(bimp_adjoint* a) {
   if (!a) return BIMP_OK;
   cudaSetDevice(a->device);
   if (a->mem) cudaFree(a->mem);
+  if (a->keep) cudaFree(a->keep);
   delete a;
   return BIMP_OK;
 }
 
 int bimp_adjoint_num_scales(const bimp_adjoint* a) { return a ? a->nScales : 0; }
 
-size_t bimp_adjoint_device_bytes(const bimp_adjoint* a) { return a ? a->bytes : 0; }
+size_t bimp_adjoint_device_bytes(const bimp_adjoint* a) { return a ? a->bytes + a->keepBytes : 0; }
 
 int bimp_adjoint_mask_layout(const bimp_adjoint* a, int scale, int* data_w, int* data_h, size_t* offset,
                              size_t* mask_stride) {

@@ -9,8 +9,8 @@
 //                       element (r+1, 0): its gradient is kept aside and
 //                       added there by the tile backward)
 //   k_gabor_tiles_bwd   per tile: the image spectrum X and, per orientation,
-//                       z = e + i o recomputed as the forward computes them
-//                       (nothing of the forward's responses is stored);
+//                       z = e + i o, kept by the forward or recomputed as it
+//                       computes them;
 //                       a = dL/dC * z/|z|, A = FFT(a), alpha/rho dot products
 //                       sum dG Re(conj(A) X), and the sum of A G in the
 //                       frequency domain; one inverse transform per tile
@@ -278,21 +278,27 @@ __device__ __forceinline__ int perm128d(int k) { return 8 * (k & 15) + (k >> 4);
 // columns).  The window gradient is linear in the per-orientation spectra,
 // Re IFFT(sum_o A_o G_o), so the products are summed in the frequency domain
 // (Hermitian half, Bh) and ONE inverse transform per item replaces one per
-// orientation.  Nothing of the forward's responses is stored: per item the
-// image spectrum X is recomputed from the float level (the forward's
-// transform: full spectrum into TMEM, Hermitian half into this CTA's slot of
-// `xscratch`), and per orientation e + i o is recomputed on the valid outputs
-// by the forward's inverse passes (G read from L2 instead of staged); then
-// a = dL/dC * z/|z| (0 where |z| <= kMagFloor or outside the valid outputs),
-// A = FFT(a), the alpha/rho dot products sum dG Re(conj(A) X), and
-// Bh += (A G + conj(A G)(-k))/2.  The per-orientation coefficients G(+-k),
-// dGa, dGr come pre-gathered in the half layout (ScaleDev::bwA, bwB).
+// orientation.  Per orientation a = dL/dC * z/|z| (0 where |z| <= kMagFloor or
+// outside the valid outputs), A = FFT(a), the alpha/rho dot products
+// sum dG Re(conj(A) X), and Bh += (A G + conj(A G)(-k))/2.  The
+// per-orientation coefficients G(+-k), dGa, dGr come pre-gathered in the half
+// layout (ScaleDev::bwA, bwB).
+//
+// KEPT: z = e + i o and the tile's image spectrum X (Hermitian half) are what
+// the forward wrote (ScaleDev::Z, X), z in the order of these lanes: a block of
+// four rows is eight coalesced 16-byte loads a lane, in L2 since the orientation
+// before.  Otherwise, where the forward had no memory for them, X is
+// recomputed per item from the float level (the forward's transform: full
+// spectrum into TMEM, Hermitian half into this CTA's slot of `xscratch`) and z
+// per orientation by the forward's inverse passes (G read from L2 instead of
+// staged).  That costs 60 k + 30 k cycles per item + orientation against 43 k +
+// 24 k here and 12 bytes of memory an output: 16 images of 512 x 512 took 1680
+// us recomputed and take 1240 kept, the forward 864 us instead of 791.
 //
 // The x-passes of both directions run on the same rows, so a warp takes
 // blocks of four valid rows through all of them (inverse 8 and 16, magnitude,
 // forward 16 and 8) with no CTA barrier, its dL/dC values loaded before the
-// first; the y-passes meet at barriers of the four warps of a lane block.  Three
-// CTA barriers an orientation are left of seven.
+// first; the y-passes meet at barriers of the four warps of a lane block.
 constexpr int kBwRaw = kTile * RawWindow<true>::kPitch * 4;   // staged float window, over Bh
 constexpr int kSmemBwBh = kBwRaw > kSmemXh ? kBwRaw : kSmemXh;
 constexpr int kGaborBwdSmem = kSmemW + kSmemBwBh + kSmemTw + kSmemMaps + 32;
@@ -318,6 +324,7 @@ struct BwEntries {
   float2 X[4];
 };
 
+template <bool KEPT>
 __global__ void __launch_bounds__(kTileThreads, 1)
 k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__ work, int nwork,
                   float2* __restrict__ xscratch, double* __restrict__ gparams) {
@@ -333,7 +340,7 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
   const uint32_t barW = smem_u32(bars);
   float2* Nyq = Bh;                                 // forward transform only (Bh is cleared after it)
   float* rawBuf = reinterpret_cast<float*>(Bh);     // the staged window, before Bh and Nyq
-  float2* __restrict__ Xs = xscratch + (size_t)blockIdx.x * kSpecHalf;
+  float2* Xs = KEPT ? nullptr : xscratch + (size_t)blockIdx.x * kSpecHalf;
   const int t = threadIdx.x;
   if (t < 8 * 17) {
     const int n1 = t / 17, k2 = t % 17;
@@ -343,11 +350,11 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
     mbar_init(barW, kTileThreads / 32);
     fence_mbar_init();
   }
-  if ((t >> 5) == 0) tmem_alloc_warp(smem_u32(tmemSlot));
+  if (!KEPT && (t >> 5) == 0) tmem_alloc_warp(smem_u32(tmemSlot));
   tmem_fence_before();
   __syncthreads();
   tmem_fence_after();
-  const uint32_t tlane = *tmemSlot + ((uint32_t)((t >> 5) & 3) << 21);
+  const uint32_t tlane = KEPT ? 0u : *tmemSlot + ((uint32_t)((t >> 5) & 3) << 21);
   const int h = t >> 7, pcol = PadLayout::col(t & 127);   // row group, this lane's column
   const int warp = t >> 5, quad = warp & 3, lane = t & 31;
   uint32_t phW = 0;
@@ -363,22 +370,41 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
     // rows and columns of the tile's valid outputs inside the map
     const int Vr = min(V, sd->cRows - R0), xHi = min(kX + V, sd->cCols - C0 + kX);
     const int cPitch = sd->cPitch;
+    const float4* zTile = nullptr;   // KEPT: this lane's elements of orientation 0's first block
+    size_t zOri = 0;                 // and from one orientation to the next
+    if constexpr (KEPT) {
+      const int cb = kept_column_blocks(*sd);
+      zOri = (size_t)sd->tilesX * cb * (kKeptBlock / 2);
+      zTile = reinterpret_cast<const float4*>(sd->Z + ((size_t)tx * cb + ty * kept_tile_blocks(V)) * kKeptBlock) + lane;
+      Xs = sd->X + (size_t)item.tile * kSpecHalf;
+    }
+    // into L2, before orientation o's x-passes: its kept responses (the pairs
+    // up to the last valid output) and its block of dL/dC
+    auto prefetch_orientation = [&](int o) {
+      if constexpr (KEPT) {
+        if (t < (Vr + 3) >> 2) {
+          const float4* z = zTile - lane + o * zOri + (size_t)t * (kKeptBlock / 2);
+          asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(z), "r"(512 * ((xHi + 15) >> 4)) : "memory");
+        }
+      }
+      prefetch_block(sd->gC + (size_t)o * sd->cStride, cPitch, R0, Vr, C0, C0 + xHi - kX, t);
+    };
     __syncthreads();   // previous tile finished with every buffer
-    raw_chunks_load<true>(sd, R0, C0, rawBuf, t);
+    if constexpr (!KEPT) raw_chunks_load<true>(sd, R0, C0, rawBuf, t);
     if (t < kTile) rmap[t] = (short)window_src(R0 - kX, t, sd->fftH, sd->dataH, kX);
     else if (t < 2 * kTile) cmap[t - kTile] = (short)window_src(C0 - kX, t - kTile, sd->fftW, sd->dataW, kX);
-    float* raw = rawBuf + ((C0 - kX) & 3);
-    {
+    prefetch_orientation(oB);
+    if constexpr (!KEPT) {
+      float* raw = rawBuf + ((C0 - kX) & 3);
       const WindowSpan<true> span(sd, C0);
       if (!span.all()) raw_window_copy<true>(sd, R0, C0, raw, span.iA, span.iB, t);
+      cp_async_wait();
+      __syncthreads();
+      tile_forward_spectrum<true, true, PadLayout>(raw, W, Nyq, tw, tlane, Xs, t, [] {});
+      tmem_fence_before();
+      __syncthreads();   // the half spectrum in W / Bh is dead from here; X complete in TMEM and Xs
+      tmem_fence_after();
     }
-    prefetch_block(sd->gC + (size_t)oB * sd->cStride, cPitch, R0, Vr, C0, C0 + xHi - kX, t);
-    cp_async_wait();
-    __syncthreads();
-    tile_forward_spectrum<true, true, PadLayout>(raw, W, Nyq, tw, tlane, Xs, t, [] {});
-    tmem_fence_before();
-    __syncthreads();   // the half spectrum in W / Bh is dead from here; X complete in TMEM and Xs
-    tmem_fence_after();
     for (int j = t; j < kTile * kXhCols; j += kTileThreads) Bh[j] = make_float2(0.f, 0.f);
     // x-pass lanes keep column group n1 = t mod 8: bit n2 says whether output
     // x = n1 + 8 n2 is valid and inside the map; bit n2 + 16 it of yMask the
@@ -391,60 +417,71 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
       yMask |= (y >= kX && y < kX + Vr ? 1u : 0u) << n2 | (y + 4 >= kX && y + 4 < kX + Vr ? 0x10000u : 0u) << n2;
     }
     for (int o = oB; o < oE; ++o) {
-      // I1: y-dim pass B' with the spectrum product X * G_o (TMEM in, TMEM out)
-      {
-        // all of the thread's G under way before its first use
-        const float4* Go = reinterpret_cast<const float4*>(sd->G + (size_t)o * kSpecFloats) + gpos(8 * h, t & 127) / 4;
-        float4 g0[4], g1[4];
+      if constexpr (!KEPT) {
+        // I1: y-dim pass B' with the spectrum product X * G_o (TMEM in, TMEM out)
+        {
+          // all of the thread's G under way before its first use
+          const float4* Go = reinterpret_cast<const float4*>(sd->G + (size_t)o * kSpecFloats) + gpos(8 * h, t & 127) / 4;
+          float4 g0[4], g1[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          g0[q] = __ldg(Go + 8 * q * kTile);
-          g1[q] = __ldg(Go + (8 * q + 1) * kTile);
+          for (int q = 0; q < 4; ++q) {
+            g0[q] = __ldg(Go + 8 * q * kTile);
+            g1[q] = __ldg(Go + (8 * q + 1) * kTile);
+          }
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int k2 = h + 4 * q;
+            float2 v[8];
+            tmem_load8(tlane + 16 * k2, v);
+            const float ga[8] = {g0[q].x, g0[q].y, g0[q].z, g0[q].w, g1[q].x, g1[q].y, g1[q].z, g1[q].w};
+            float2 twr[8];
+#pragma unroll
+            for (int n1 = 1; n1 < 8; ++n1) twr[n1] = tw[n1 * 17 + k2];
+#pragma unroll
+            for (int k1 = 0; k1 < 8; ++k1) v[k1] = c_scale(v[k1], ga[k1]);
+            dft8<true>(v);
+#pragma unroll
+            for (int n1 = 0; n1 < 8; ++n1)
+              tmem_store1(tlane + kTmemY + 2 * (16 * n1 + k2), n1 ? c_mulc(v[n1], twr[n1]) : v[0]);
+          }
         }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int k2 = h + 4 * q;
-          float2 v[8];
-          tmem_load8(tlane + 16 * k2, v);
-          const float ga[8] = {g0[q].x, g0[q].y, g0[q].z, g0[q].w, g1[q].x, g1[q].y, g1[q].z, g1[q].w};
-          float2 twr[8];
-#pragma unroll
-          for (int n1 = 1; n1 < 8; ++n1) twr[n1] = tw[n1 * 17 + k2];
-#pragma unroll
-          for (int k1 = 0; k1 < 8; ++k1) v[k1] = c_scale(v[k1], ga[k1]);
-          dft8<true>(v);
-#pragma unroll
-          for (int n1 = 0; n1 < 8; ++n1)
-            tmem_store1(tlane + kTmemY + 2 * (16 * n1 + k2), n1 ? c_mulc(v[n1], twr[n1]) : v[0]);
+        tmem_wait_st();
+        tmem_fence_before();
+        named_barrier(1 + quad, kTileThreads / 4);   // the lane block's first y-pass is complete
+        tmem_fence_after();
+        if (o > oB) {   // every warp is done with the previous orientation's accumulation
+          mbar_wait(barW, phW);
+          phW ^= 1u;
+          __syncwarp();
         }
-      }
-      tmem_wait_st();
-      tmem_fence_before();
-      named_barrier(1 + quad, kTileThreads / 4);   // the lane block's first y-pass is complete
-      tmem_fence_after();
-      if (o > oB) {   // every warp is done with the previous orientation's accumulation
-        mbar_wait(barW, phW);
-        phW ^= 1u;
-        __syncwarp();
-      }
-      // I2: y-dim pass A' -> natural y; rows outside the valid band are zero
-      // (a is zero there, and the transform of a below reads every row)
+        // I2: y-dim pass A' -> natural y; rows outside the valid band are zero
+        // (a is zero there, and the transform of a below reads every row)
 #pragma unroll
-      for (int it = 0; it < 2; ++it) {
-        const int n1 = h + 4 * it;
-        float2 v[16];
-        tmem_load16(tlane + kTmemY + 32 * n1, v);
-        dft16<true>(v);
+        for (int it = 0; it < 2; ++it) {
+          const int n1 = h + 4 * it;
+          float2 v[16];
+          tmem_load16(tlane + kTmemY + 32 * n1, v);
+          dft16<true>(v);
 #pragma unroll
-        for (int n2 = 0; n2 < 16; ++n2) {
-          W[widx(n1 + 8 * n2, pcol)] = (yMask >> (n2 + 16 * it)) & 1u ? v[n2] : make_float2(0.f, 0.f);
+          for (int n2 = 0; n2 < 16; ++n2) {
+            W[widx(n1 + 8 * n2, pcol)] = (yMask >> (n2 + 16 * it)) & 1u ? v[n2] : make_float2(0.f, 0.f);
+          }
         }
+        tmem_fence_before();
+        __syncthreads();
+        tmem_fence_after();
       }
-      tmem_fence_before();
-      __syncthreads();
-      tmem_fence_after();
-      if (o + 1 < oE)
-        prefetch_block(sd->gC + (size_t)(o + 1) * sd->cStride, cPitch, R0, Vr, C0, C0 + xHi - kX, t);
+      if (o + 1 < oE) prefetch_orientation(o + 1);
+      // KEPT: W is free when every warp is done with the previous
+      // orientation's accumulation
+      auto wait_w = [&] {
+        if (KEPT && o > oB) {
+          mbar_wait(barW, phW);
+          phW ^= 1u;
+          __syncwarp();
+        }
+      };
+      if (KEPT && 4 * warp >= Vr) wait_w();   // (a warp without rows)
       // The x-passes, four valid rows to a warp at a time: I3 (x-dim pass B');
       // I4 (pass A': z = e + i o at the row's outputs x = n1 + 8 n2),
       // a = dL/dC * z/|z| (|z| as the forward computed it) and the forward
@@ -469,28 +506,41 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
             for (int n2 = 0; n2 < 16; ++n2)
               if (n2 == (kX >> 3)) gcv[n2] += add;
           }
-          {
-            float2 twr[8];
+          float2 v[16];
+          if constexpr (KEPT) {
+            const float4* z = zTile + o * zOri + (size_t)(r0 >> 2) * (kKeptBlock / 2);
 #pragma unroll
-            for (int m = 1; m < 8; ++m) twr[m] = tw[m * 17 + k2];
-#pragma unroll 1
-            for (int q = r0 + (lane >> 4); q < min(Vr, r0 + 4); q += 2) {
-              float2* wr = W + widx(kX + q, 8 * k2);
-              float2 v[8];
-#pragma unroll
-              for (int k1 = 0; k1 < 8; ++k1) v[k1] = wr[k1];
-              dft8<true>(v);
-#pragma unroll
-              for (int m = 0; m < 8; ++m) wr[m] = m ? c_mulc(v[m], twr[m]) : v[0];
+            for (int p = 0; p < 8; ++p) {
+              const float4 zz = r < Vr && 16 * p + 15 >= kX && 16 * p < xHi ? __ldcs(z + 32 * p) : make_float4(0.f, 0.f, 0.f, 0.f);
+              v[2 * p] = make_float2(zz.x, zz.y);
+              v[2 * p + 1] = make_float2(zz.z, zz.w);
             }
+            if (r0 == 4 * warp) wait_w();
+          } else {
+            {
+              float2 twr[8];
+#pragma unroll
+              for (int m = 1; m < 8; ++m) twr[m] = tw[m * 17 + k2];
+#pragma unroll 1
+              for (int q = r0 + (lane >> 4); q < min(Vr, r0 + 4); q += 2) {
+                float2* wr = W + widx(kX + q, 8 * k2);
+                float2 v[8];
+#pragma unroll
+                for (int k1 = 0; k1 < 8; ++k1) v[k1] = wr[k1];
+                dft8<true>(v);
+#pragma unroll
+                for (int m = 0; m < 8; ++m) wr[m] = m ? c_mulc(v[m], twr[m]) : v[0];
+              }
+            }
+            __syncwarp();
           }
-          __syncwarp();
           if (r < Vr) {
             float2* wr = W + widx(kX + r, n1);
-            float2 v[16];
+            if constexpr (!KEPT) {
 #pragma unroll
-            for (int m = 0; m < 16; ++m) v[m] = wr[9 * m];
-            dft16<true>(v);
+              for (int m = 0; m < 16; ++m) v[m] = wr[9 * m];
+              dft16<true>(v);
+            }
 #pragma unroll
             for (int n2 = 0; n2 < 16; ++n2) {
               // |z| as the forward computes it (s * rsqrt(s)); 1/|z| is the
@@ -535,7 +585,11 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
         float2* col = W + widx(n1, pcol);
         float2 v[16];
 #pragma unroll
-        for (int m = 0; m < 16; ++m) v[m] = col[8 * m * kWPitch];
+        for (int m = 0; m < 16; ++m) {
+          // KEPT: the rows outside the valid band are left as they were
+          const bool rowIn = !KEPT || ((yMask >> (m + 16 * it)) & 1u);
+          v[m] = rowIn ? col[8 * m * kWPitch] : make_float2(0.f, 0.f);
+        }
         dft16<false>(v);
         float2 twr[16];
 #pragma unroll
@@ -554,7 +608,7 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
           const int j = (pr + 8 * (r0 + u)) * kXhCols + sl;
           e.c4[u] = __ldg(cA + j);
           e.c2[u] = __ldg(cB + j);
-          e.X[u] = Xs[j];   // written by this CTA for this item: a coherent load
+          e.X[u] = KEPT ? __ldg(Xs + j) : Xs[j];   // recomputed: written by this CTA for this item, a coherent load
         }
       };
       BwEntries next;
@@ -692,7 +746,7 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
   tmem_fence_before();
   __syncthreads();
   tmem_fence_after();
-  if ((t >> 5) == 0) tmem_dealloc_warp(*tmemSlot);
+  if (!KEPT && (t >> 5) == 0) tmem_dealloc_warp(*tmemSlot);
   block_add_double(accA, gparams + 0);
   block_add_double(accR, gparams + 1);
 }

@@ -11,6 +11,12 @@
 
 #include "bimp_b200.h"
 
+#ifdef __CUDACC__
+#define BIMP_HOST_DEVICE __host__ __device__
+#else
+#define BIMP_HOST_DEVICE
+#endif
+
 namespace bimp_b200 {
 
 constexpr int kNumOri = 8;
@@ -68,7 +74,7 @@ struct ScaleDev {
   // differentiable path (float pyramid, saved responses, adjoint buffers)
   const float* lvlF;      // float level (X scale), lvlPitchF floats per row
   int lvlPitchF;
-  float2* Z;              // saved e + i o, C layout in float2
+  float2* Z;              // saved e + i o: C layout in float2 (line/edge detection), kept_z_at order (adjoint), or null
   const float* M;         // loss weights, dataH x dataW (row pitch dataW)
   float* gC;              // d loss / d complex cell, C layout
   float* gWrap;           // fftW == dataW: d loss / d window (r, dataW), kNumOri x (dataH + 1)
@@ -76,8 +82,19 @@ struct ScaleDev {
   unsigned int* bits;     // ReLU states, 4 bits per orientation, dataH x dPitch
   const float4* bwA;      // per orientation, kSpecHalf entries {G(k), G(-k), dGa(k), dGr(k)}
   const float2* bwB;      //   {dGa(-k), dGr(-k)}; dG* = spectra of d taps / d alpha, d rho
-  int pad[2];             // to a multiple of 16 bytes: the tile kernel copies records as 16-byte words
+  float2* X;              // kept image spectra, kSpecHalf per tile, or null.  (The record's size is a multiple of
+                          // 16 bytes: the tile kernel copies records as 16-byte words)
 };
+
+// The adjoint's kept responses: per orientation and tile column, the column's
+// blocks of four valid rows from the top (tile row ty starts at block ty *
+// blocks(V)); a block holds, for n2 = 2 p, 2 p + 1 (p < 8) and each lane (row
+// lane / 8, n1 = lane mod 8), the outputs x = n1 + 8 n2 as the x-passes hold them.
+constexpr int kKeptBlock = 4 * kTile;   // float2 of a block
+BIMP_HOST_DEVICE inline int kept_tile_blocks(int rows) { return (rows + 3) >> 2; }
+BIMP_HOST_DEVICE inline int kept_column_blocks(const ScaleDev& d) {
+  return (d.tilesY - 1) * kept_tile_blocks(d.V) + kept_tile_blocks(d.cRows - (d.tilesY - 1) * d.V);
+}
 
 // Stencil offset sets of the two level wavelengths the default bank uses
 // (lambda ~ 4 and ~ 5.657 at every pyramid level); scales whose offsets equal

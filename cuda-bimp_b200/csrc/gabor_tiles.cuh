@@ -364,7 +364,7 @@ __device__ __forceinline__ void raw_window_copy(const ScaleDev* sd, int R0, int 
 // h + 4 q, of its lane's column (h = t / 128).  W: work buffer, of
 // which the part behind the 64 packed rows (LY::kHalf; `raw` may lie there)
 // later holds the half spectrum; Nyq its column kx = 64.  SAVE_X also writes the
-// Hermitian half to global memory, Xs[py * kXhCols + slot].
+// Hermitian half to global memory, Xs[py * kXhCols + slot], where Xs is given.
 template <bool FLT, bool SAVE_X, class LY, class Hook>
 __device__ __forceinline__ void tile_forward_spectrum(const typename RawWindow<FLT>::T* raw, float2* W, float2* Nyq,
                                                       const float2* tw, uint32_t tlane, float2* __restrict__ Xs, int t,
@@ -466,7 +466,7 @@ __device__ __forceinline__ void tile_forward_spectrum(const typename RawWindow<F
       for (int k1 = 0; k1 < 8; ++k1) x[k1].y *= sign;
       tmem_store8(tlane + 16 * k2, x);
       if constexpr (SAVE_X) {
-        if (!hc.conj) {
+        if (Xs && !hc.conj) {
 #pragma unroll
           for (int k1 = 0; k1 < 8; ++k1) Xs[(8 * k2 + k1) * kXhCols + hc.slot] = x[k1];
         }
@@ -573,7 +573,9 @@ k_gabor_tiles(const ScaleDev* __restrict__ sds, const TileWork* __restrict__ wor
       if (!span.all()) raw_window_copy<FLT>(sd, R0, C0, raw, span.iA, span.iB, t);
       cp_async_wait();
       __syncthreads();
-      tile_forward_spectrum<FLT, false, PadLayout>(raw, W, Nyq, tw, tlane, nullptr, t, [] {});
+      // the adjoint keeps the spectrum of every tile (orientation 0's item writes it)
+      float2* Xk = SAVE_Z && oB == 0 ? sd->X + (size_t)item.tile * kSpecHalf : nullptr;
+      tile_forward_spectrum<FLT, SAVE_Z, PadLayout>(raw, W, Nyq, tw, tlane, Xk, t, [] {});
     } else {
       uint8_t* raw = rawG + ((C0 - kX) & 15);
       const WindowSpan<FLT> span(sd, C0);
@@ -748,7 +750,17 @@ k_gabor_tiles(const ScaleDev* __restrict__ sds, const TileWork* __restrict__ wor
                 }
               }
             }
-            if constexpr (SAVE_Z) {   // e + i o, laid out as the magnitudes
+            if constexpr (SAVE_Z && FLT) {   // e + i o, as these lanes hold it
+              const int bpt = kept_tile_blocks(V);
+              float4* z = reinterpret_cast<float4*>(
+                              lds_now(&sd->Z) + (((size_t)o * sd->tilesX + tx) * kept_column_blocks(*sd) + ty * bpt + (r0 >> 2)) * kKeptBlock) +
+                          lane;
+#pragma unroll
+              for (int p = 0; p < 8; ++p)
+                if (16 * p + 15 >= kX && 16 * p < xHi)
+                  __stcs(z + 32 * p, make_float4(v[2 * p].x, v[2 * p].y, v[2 * p + 1].x, v[2 * p + 1].y));
+            }
+            if constexpr (SAVE_Z && !FLT) {   // e + i o, laid out as the magnitudes
               float2* __restrict__ z = sd->Z + (dst - sd->C);
               const int cCols = sd->cCols, cRows = sd->cRows;
 #pragma unroll

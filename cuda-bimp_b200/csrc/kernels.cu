@@ -1326,7 +1326,9 @@ cudaError_t configure_kernels() {
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_stencil<kStencilD>, big, (int)stencil_smem_bytes());
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_stencil<kStencilDS>, big, (int)stencil_smem_bytes());
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_stencil<kStencilAdj>, big, (int)stencil_smem_bytes());
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_gabor_tiles_bwd, big, (int)kGaborBwdSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_gabor_tiles_bwd<false>, big, (int)kGaborBwdSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_gabor_tiles_bwd<true>, big, (int)kGaborBwdSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_gabor_tiles<true, true>, big, (int)gabor_smem_bytes());
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_gabor_tiles_ws<false>, big, (int)kWsSmem);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_gabor_tiles_ws<true>, big, (int)kWsSmem);
   if (e != cudaSuccess) return e;
@@ -1376,9 +1378,11 @@ void launch_gabor(const ScaleDev* d_sd, const TileWork* d_work, int nwork, int g
               d_fault);
 }
 void launch_gabor_flt(const ScaleDev* d_sd, const TileWork* d_work, int nwork, int grid, unsigned int* d_fault,
-                      cudaStream_t s, bool pipelined) {
+                      cudaStream_t s, bool pipelined, bool keep) {
   if (nwork <= 0) return;
-  if (pipelined)
+  if (keep)
+    k_gabor_tiles<true, true><<<grid, kTileThreads, gabor_smem_bytes(), s>>>(d_sd, d_work, nwork, d_fault);
+  else if (pipelined)
     k_gabor_tiles_ws<true><<<grid, kTileThreads, kWsSmem, s>>>(d_sd, d_work, nwork);
   else
     k_gabor_tiles<true, false><<<grid, kTileThreads, gabor_smem_bytes(), s>>>(d_sd, d_work, nwork, d_fault);
@@ -1406,10 +1410,9 @@ void launch_stencil_bwd(const ScaleDev* d_sd, const int2* d_work, int nwork, cud
 }
 
 void launch_gabor_bwd(const ScaleDev* d_sd, const TileWork* d_work, int nwork, int grid, float2* d_xscratch,
-                      double* d_gparams, cudaStream_t s) {
-  if (nwork > 0)
-    k_gabor_tiles_bwd<<<grid, kTileThreads, kGaborBwdSmem, s>>>(d_sd, d_work, nwork, d_xscratch,
-                                                                                 d_gparams);
+                      double* d_gparams, cudaStream_t s, bool kept) {
+  auto k = kept ? k_gabor_tiles_bwd<true> : k_gabor_tiles_bwd<false>;
+  if (nwork > 0) k<<<grid, kTileThreads, kGaborBwdSmem, s>>>(d_sd, d_work, nwork, d_xscratch, d_gparams);
 }
 void launch_stencil(const ScaleDev* d_sd, const int2* d_work, int nwork, unsigned int* d_fault, cudaStream_t s,
                     int mode, bool pdl, double* d_loss, double* d_gparams) {

@@ -99,9 +99,9 @@ void launch_nms(const ScaleDev* d_sd, const int2* d_rows, int nrows, int* d_coun
 void launch_pyr_f(const PyrJobF* d_jobs, int njobs, int maxW, int maxH, cudaStream_t s);
 void launch_pyr_f_adj(const PyrJobF* d_jobs, int njobs, int maxW, int maxH, cudaStream_t s);
 // differentiable forward: the tile kernel on the float levels (`grid`
-// persistent CTAs)
+// persistent CTAs); keep: it also writes ScaleDev::Z and X for the backward
 void launch_gabor_flt(const ScaleDev* d_sd, const TileWork* d_work, int nwork, int grid, unsigned int* d_fault,
-                      cudaStream_t s, bool pipelined);
+                      cudaStream_t s, bool pipelined, bool keep);
 // detection-path tile kernel that also keeps e + i o (ScaleDev::Z) for the
 // line/edge detector; one CTA per work item
 void launch_gabor_keep_z(const ScaleDev* d_sd, const TileWork* d_work, int nwork, unsigned int* d_fault,
@@ -110,9 +110,10 @@ void launch_gabor_keep_z(const ScaleDev* d_sd, const TileWork* d_work, int nwork
 void launch_detect_le(const ScaleDev* d_sd, int dataW, int dataH, const float* d_ch, int chLd, float* d_result,
                       float* d_ori, int8_t* d_type, int ld, cudaStream_t s);
 void launch_stencil_bwd(const ScaleDev* d_sd, const int2* d_work, int nwork, cudaStream_t s);
-// tile backward, recomputing the responses; `grid` persistent CTAs,
-// d_xscratch holds grid x kSpecHalf float2 (one tile spectrum per CTA)
+// tile backward, from the kept responses or recomputing them; `grid` persistent
+// CTAs; to recompute, d_xscratch holds grid x kSpecHalf float2 (one tile
+// spectrum per CTA)
 void launch_gabor_bwd(const ScaleDev* d_sd, const TileWork* d_work, int nwork, int grid, float2* d_xscratch,
-                      double* d_gparams, cudaStream_t s);
+                      double* d_gparams, cudaStream_t s, bool kept);
 
 }  // namespace bimp_b200

@@ -21,7 +21,9 @@
  * (exactly flat image regions give |e + i o| = 0 up to rounding, where the
  * magnitude has no derivative; the value assumes images on the [0, 1] scale).
  * The forward keeps the complex responses and each tile's image spectrum
- * for the backward.
+ * for the backward where the adjoint got the memory for them when it was
+ * created (up to 8 GiB and an eighth of the device's free memory); otherwise
+ * the backward recomputes them, with the same results.
  */
 #ifndef BIMP_B200_ADJOINT_H
 #define BIMP_B200_ADJOINT_H
