@@ -291,9 +291,9 @@ __device__ __forceinline__ int perm128d(int k) { return 8 * (k & 15) + (k >> 4);
 // recomputed per item from the float level (the forward's transform: full
 // spectrum into TMEM, Hermitian half into this CTA's slot of `xscratch`) and z
 // per orientation by the forward's inverse passes (G read from L2 instead of
-// staged).  That costs 60 k + 30 k cycles per item + orientation against 43 k +
-// 24 k here and 12 bytes of memory an output: 16 images of 512 x 512 took 1680
-// us recomputed and take 1240 kept, the forward 864 us instead of 791.
+// staged).  That costs 60 k + 30 k cycles per item + orientation against 40 k +
+// 22 k here and 12 bytes of memory an output: 16 images of 512 x 512 took 1680
+// us recomputed and take 1165 kept, the forward 864 us instead of 791.
 //
 // The x-passes of both directions run on the same rows, so a warp takes
 // blocks of four valid rows through all of them (inverse 8 and 16, magnitude,
@@ -306,22 +306,26 @@ static_assert(kGaborBwdSmem <= 232448, "tile backward exceeds the 227 KB shared-
 
 // Prefetch into L2 of the block of dL/dC that one orientation's magnitude pass
 // reads: rows [R0, R0 + rows), columns [x0, x1) of a map with row pitch `pitch`
-// floats (rows start on 128-byte lines).  One 128-byte line per thread and
-// step; addresses stay inside the map.
+// floats (rows start on 128-byte lines).  Four threads a row take its lines (at
+// most five); addresses stay inside the map.
 __device__ __forceinline__ void prefetch_block(const float* base, int pitch, int R0, int rows, int x0, int x1, int t) {
-  if (rows <= 0 || x1 <= x0) return;
-  const int l0 = x0 >> 5, nl = ((x1 - 1) >> 5) - l0 + 1;   // 32 floats per line
-  for (int i = t; i < rows * nl; i += kTileThreads) {
-    const int r = i / nl, l = l0 + (i - r * nl);
+  static_assert(kTileThreads == 4 * kTile, "four threads a row");
+  const int r = t >> 2, end = (x1 + 31) >> 5;   // 32 floats per line
+  if (r >= rows) return;
+  for (int l = (x0 >> 5) + (t & 3); l < end; l += 4)
     asm volatile("prefetch.global.L2 [%0];" ::"l"(base + (size_t)(R0 + r) * pitch + 32 * l));
-  }
+}
+
+// Adds four consecutive floats (16-byte aligned).
+__device__ __forceinline__ void red_add4(float* p, float4 v) {
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
 }
 
 // The coefficients and image spectrum of four entries of the accumulation.
 struct BwEntries {
   float4 c4[4];   // G(k), G(-k), dGa(k), dGr(k)
   float2 c2[4];   // dGa(-k), dGr(-k)
-  float2 X[4];
+  float2 X[4];    // (recomputed: from global memory)
 };
 
 template <bool KEPT>
@@ -350,11 +354,11 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
     mbar_init(barW, kTileThreads / 32);
     fence_mbar_init();
   }
-  if (!KEPT && (t >> 5) == 0) tmem_alloc_warp(smem_u32(tmemSlot));
+  if ((t >> 5) == 0) tmem_alloc_warp(smem_u32(tmemSlot));
   tmem_fence_before();
   __syncthreads();
   tmem_fence_after();
-  const uint32_t tlane = KEPT ? 0u : *tmemSlot + ((uint32_t)((t >> 5) & 3) << 21);
+  const uint32_t tlane = *tmemSlot + ((uint32_t)((t >> 5) & 3) << 21);
   const int h = t >> 7, pcol = PadLayout::col(t & 127);   // row group, this lane's column
   const int warp = t >> 5, quad = warp & 3, lane = t & 31;
   uint32_t phW = 0;
@@ -404,6 +408,19 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
       tmem_fence_before();
       __syncthreads();   // the half spectrum in W / Bh is dead from here; X complete in TMEM and Xs
       tmem_fence_after();
+    }
+    if constexpr (KEPT) {
+      // this thread's 16 entries of X for the accumulation, in its own lane of
+      // the tensor memory (32 columns a warp): read from L2 with the
+      // coefficients they were a quarter of that phase's traffic
+#pragma unroll
+      for (int r0 = 0; r0 < 16; r0 += 8) {
+        float2 x[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) x[u] = __ldg(Xs + ((t >> 6) + 8 * (r0 + u)) * kXhCols + (t & 63));
+        tmem_store8(tlane + 32 * (warp >> 2) + 2 * r0, x);
+      }
+      tmem_wait_st();
     }
     for (int j = t; j < kTile * kXhCols; j += kTileThreads) Bh[j] = make_float2(0.f, 0.f);
     // x-pass lanes keep column group n1 = t mod 8: bit n2 says whether output
@@ -608,7 +625,7 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
           const int j = (pr + 8 * (r0 + u)) * kXhCols + sl;
           e.c4[u] = __ldg(cA + j);
           e.c2[u] = __ldg(cB + j);
-          e.X[u] = KEPT ? __ldg(Xs + j) : Xs[j];   // recomputed: written by this CTA for this item, a coherent load
+          if constexpr (!KEPT) e.X[u] = Xs[j];   // written by this CTA for this item: a coherent load
         }
       };
       BwEntries next;
@@ -636,20 +653,22 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
         const int kx = half_group(sl) + 16 * (sl & 3);
         const float2* W1 = W + widx(pr, perm128d(kx));
         const float2* W2 = W + widx(0, perm128d((kTile - kx) & 127));
+        float2 X8[8];
 #pragma unroll
         for (int r0 = 0; r0 < 16; r0 += 4) {
           BwEntries e = next;
           if (r0 + 4 < 16) fetch(r0 + 4, next);
+          if (KEPT && r0 % 8 == 0) tmem_load8(tlane + 32 * (warp >> 2) + 2 * r0, X8);
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
             const int py = pr + 8 * (r0 + u), j = py * kXhCols + sl;
             const int ky = 16 * (py & 7) + (py >> 3);
             const float2 A1 = W1[8 * (r0 + u) * kWPitch], A2 = W2[perm128d((kTile - ky) & 127) * kWPitch];
-            const float2 bb = Bh[j];
+            const float2 bb = Bh[j], X = KEPT ? X8[(r0 & 4) + u] : e.X[u];
             Bh[j] = make_float2(fmaf(0.5f * e.c4[u].x, A1.x, fmaf(0.5f * e.c4[u].y, A2.x, bb.x)),
                                 fmaf(0.5f * e.c4[u].x, A1.y, fmaf(-0.5f * e.c4[u].y, A2.y, bb.y)));
-            const float re1 = A1.x * e.X[u].x + A1.y * e.X[u].y;   // Re(conj(A(k)) X(k))
-            const float re2 = A2.x * e.X[u].x - A2.y * e.X[u].y;   // Re(conj(A(-k)) conj(X(k)))
+            const float re1 = A1.x * X.x + A1.y * X.y;   // Re(conj(A(k)) X(k))
+            const float re2 = A2.x * X.x - A2.y * X.y;   // Re(conj(A(-k)) conj(X(k)))
             sa = fmaf(e.c4[u].z, re1, fmaf(e.c2[u].x, re2, sa));
             sr = fmaf(e.c4[u].w, re1, fmaf(e.c2[u].y, re2, sr));
           }
@@ -715,6 +734,10 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
     {
       float* __restrict__ gl = sd->gLvl;
       const int gp = sd->lvlPitchF, k2 = lane & 15, n1 = lane & 7;
+      // window columns [iA, iB) are consecutive data columns; quads of them
+      // start 16-byte aligned in the level `lead` columns before the window
+      // (level rows start 16-byte aligned, their pitch is a multiple of 32)
+      const int iA = min(max(kX - C0, 0), kTile), iB = max(iA, min(kTile, sd->dataW - (C0 - kX))), lead = (C0 - kX) & 3;
 #pragma unroll 1
       for (int r0 = 8 * warp; r0 < 8 * warp + 8; r0 += 4) {
 #pragma unroll 1
@@ -734,19 +757,66 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
 #pragma unroll
         for (int m = 0; m < 16; ++m) v[m] = wr[9 * m];
         dft16<true>(v);
-        float* row = gl + (size_t)rmap[y] * gp;
+        // the row's values in natural order over its own (read) elements, from
+        // float `lead` of it on, then four at a time into the level.  (Rows two
+        // apart start 8 floats further on: their 4 x 8 stores hit all banks.)
+        __syncwarp();
+        {
+          float* out = reinterpret_cast<float*>(W + widx(y, 0)) + 4 * (y & 2) + lead + n1;
 #pragma unroll
-        for (int n2 = 0; n2 < 16; ++n2) {
-          const float g = v[n2].x;
-          if (g != 0.f) atomicAdd(row + cmap[n1 + 8 * n2], kFloatLevelScale * g);
+          for (int n2 = 0; n2 < 16; ++n2) out[8 * n2] = kFloatLevelScale * v[n2].x;
         }
+        __syncwarp();
+#pragma unroll 1
+        for (int i = 0; i < 5; ++i) {
+          // step i: quads 0..31 of row r0 + i; last: quad 32 of the four rows
+          const int yy = r0 + (i < 4 ? i : lane & 3), q = i < 4 ? lane : 32;
+          if (i == 4 && (lane >= 4 || lead == 0)) break;
+          const float* in = reinterpret_cast<const float*>(W + widx(yy, 0)) + 4 * (yy & 2);
+          float4 g = reinterpret_cast<const float4*>(in)[q];
+          const int x = 4 * q - lead;   // window column of g.x
+          if (x < iA || x >= iB) g.x = 0.f;
+          if (x + 1 < iA || x + 1 >= iB) g.y = 0.f;
+          if (x + 2 < iA || x + 2 >= iB) g.z = 0.f;
+          if (x + 3 < iA || x + 3 >= iB) g.w = 0.f;
+          if (g.x != 0.f || g.y != 0.f || g.z != 0.f || g.w != 0.f)
+            red_add4(gl + (size_t)rmap[yy] * gp + (C0 - kX + x), g);
+        }
+        // columns outside the data through the torus map, eight lanes to a
+        // row: those of the padding fall on the row's first or last element and
+        // are summed before they are added (one by one, up to 100 adds of a row
+        // to one address, the tiles at the right edge took 70 k of 290 k cycles
+        // longer than the others)
+        if (iA > 0 || iB < kTile) {
+          const float* in = reinterpret_cast<const float*>(W + widx(y, 0)) + 4 * (y & 2) + lead;
+          float* row = gl + (size_t)rmap[y] * gp;
+          const int last = sd->dataW - 1;
+          float toFirst = 0.f, toLast = 0.f;
+#pragma unroll 4
+          for (int n2 = 0; n2 < 16; ++n2) {
+            const int x = n1 + 8 * n2;
+            const float g = x < iA || x >= iB ? in[x] : 0.f;
+            const int c = cmap[x];
+            if (c == last) toLast += g;
+            else if (c == 0) toFirst += g;
+            else if (g != 0.f) atomicAdd(row + c, g);
+          }
+#pragma unroll
+          for (int d = 4; d > 0; d >>= 1) {
+            toFirst += __shfl_xor_sync(0xffffffffu, toFirst, d);
+            toLast += __shfl_xor_sync(0xffffffffu, toLast, d);
+          }
+          if (n1 == 0 && toFirst != 0.f) atomicAdd(row, toFirst);
+          if (n1 == 1 && toLast != 0.f) atomicAdd(row + last, toLast);
+        }
+        __syncwarp();
       }
     }
   }
   tmem_fence_before();
   __syncthreads();
   tmem_fence_after();
-  if (!KEPT && (t >> 5) == 0) tmem_dealloc_warp(*tmemSlot);
+  if ((t >> 5) == 0) tmem_dealloc_warp(*tmemSlot);
   block_add_double(accA, gparams + 0);
   block_add_double(accR, gparams + 1);
 }

@@ -24,9 +24,10 @@ constexpr TileCost kForwardCost = {1.4, 0.481, 0.0741};
 // Backward (16 x 512 x 512, residual 11 k of about 300 k cycles an item): 61 k,
 // 19.2 k, 1.68 k of 31.0 k cycles.
 constexpr TileCost kBackwardCost = {1.97, 0.62, 0.0543};
-// Backward from kept responses (same case, residual 9 k of about 220 k): 43 k,
-// 14.9 k, 1.25 k of 23.6 k cycles.
-constexpr TileCost kBackwardKeptCost = {1.82, 0.63, 0.053};
+// Backward from kept responses (between that case, 40.8 k, 13.4 k, 1.30 k, and
+// 1333 x 1001, 35.9 k, 15.3 k, 1.08 k of 22.5 k cycles; residual 10 k of about
+// 210 k).
+constexpr TileCost kBackwardKeptCost = {1.75, 0.62, 0.0535};
 
 // Balanced plan for a persistent grid of `grid` CTAs.  The (tile,
 // orientation) pairs, tile by tile in the given order, are cut into at most
