@@ -595,7 +595,10 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
         }
       }
       __syncthreads();
-      // forward y-dim passes of a, each lane's column
+      // forward y-dim passes of a, each lane's column; between them through the
+      // tensor memory as between I1 and I2 (through W they moved a third of the
+      // 11 k cycles of shared-memory traffic an orientation: 16 x 512 x 512
+      // 1165 -> 1130 us)
 #pragma unroll
       for (int it = 0; it < 2; ++it) {
         const int n1 = h + 4 * it;
@@ -608,13 +611,14 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
           v[m] = rowIn ? col[8 * m * kWPitch] : make_float2(0.f, 0.f);
         }
         dft16<false>(v);
-        float2 twr[16];
 #pragma unroll
-        for (int k2 = 0; k2 < 16; ++k2) twr[k2] = tw[n1 * 17 + k2];
-#pragma unroll
-        for (int k2 = 0; k2 < 16; ++k2) col[8 * k2 * kWPitch] = c_mul(v[k2], twr[k2]);
+        for (int k2 = 0; k2 < 16; ++k2) v[k2] = c_mul(v[k2], tw[n1 * 17 + k2]);
+        tmem_store16(tlane + kTmemY + 32 * n1, v);
       }
+      tmem_wait_st();
+      tmem_fence_before();
       named_barrier(1 + quad, kTileThreads / 4);
+      tmem_fence_after();
       // the first coefficients of the accumulation are under way during the last pass
       const float4* __restrict__ cA = sd->bwA + (size_t)o * kSpecHalf;
       const float2* __restrict__ cB = sd->bwB + (size_t)o * kSpecHalf;
@@ -634,13 +638,14 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
       for (int it = 0; it < 4; ++it) {
         float2* col = W + widx(8 * (h + 4 * it), pcol);
         float2 v[8];
-#pragma unroll
-        for (int n1 = 0; n1 < 8; ++n1) v[n1] = col[n1 * kWPitch];
+        tmem_load8_strided(tlane + kTmemY + 2 * (h + 4 * it), v);
         dft8<false>(v);
 #pragma unroll
         for (int k1 = 0; k1 < 8; ++k1) col[k1 * kWPitch] = v[k1];
       }
+      tmem_fence_before();
       __syncthreads();
+      tmem_fence_after();
       // Hermitian accumulation and the parameter dot products.  Entry j of
       // the half layout holds k = (ky, kx), kx in [0, 64]; its partner -k
       // covers the columns 65..127, so every frequency enters the dot

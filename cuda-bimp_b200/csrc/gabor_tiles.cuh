@@ -96,6 +96,22 @@ __device__ __forceinline__ void tmem_store8(uint32_t taddr, const float2 (&v)[8]
       "r"(__float_as_uint(v[6].x)), "r"(__float_as_uint(v[6].y)), "r"(__float_as_uint(v[7].x)),
       "r"(__float_as_uint(v[7].y)));
 }
+// The same for 16 complex (32 columns).
+__device__ __forceinline__ void tmem_store16(uint32_t taddr, const float2 (&v)[16]) {
+  uint32_t r[32];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    r[2 * i] = __float_as_uint(v[i].x);
+    r[2 * i + 1] = __float_as_uint(v[i].y);
+  }
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+      "%15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(taddr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]),
+      "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]),
+      "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]));
+}
 // Whole warp: each thread stores one complex (2 columns) into its own lane;
 // completion is awaited with tmem_wait_st.
 __device__ __forceinline__ void tmem_store1(uint32_t taddr, float2 v) {
@@ -130,6 +146,27 @@ __device__ __forceinline__ void tmem_load8(uint32_t taddr, float2 (&v)[8]) {
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
         "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr));
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+}
+
+// Whole warp: each thread loads 8 complex, 32 columns apart, from its own lane.
+__device__ __forceinline__ void tmem_load8_strided(uint32_t taddr, float2 (&v)[8]) {
+  uint32_t r[16];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%16];\n"
+      "tcgen05.ld.sync.aligned.32x32b.x2.b32 {%2, %3}, [%17];\n"
+      "tcgen05.ld.sync.aligned.32x32b.x2.b32 {%4, %5}, [%18];\n"
+      "tcgen05.ld.sync.aligned.32x32b.x2.b32 {%6, %7}, [%19];\n"
+      "tcgen05.ld.sync.aligned.32x32b.x2.b32 {%8, %9}, [%20];\n"
+      "tcgen05.ld.sync.aligned.32x32b.x2.b32 {%10, %11}, [%21];\n"
+      "tcgen05.ld.sync.aligned.32x32b.x2.b32 {%12, %13}, [%22];\n"
+      "tcgen05.ld.sync.aligned.32x32b.x2.b32 {%14, %15}, [%23];\n"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=&r"(r[4]), "=&r"(r[5]), "=&r"(r[6]), "=&r"(r[7]),
+        "=&r"(r[8]), "=&r"(r[9]), "=&r"(r[10]), "=&r"(r[11]), "=&r"(r[12]), "=&r"(r[13]), "=&r"(r[14]), "=&r"(r[15])
+      : "r"(taddr), "r"(taddr + 32), "r"(taddr + 64), "r"(taddr + 96), "r"(taddr + 128), "r"(taddr + 160),
+        "r"(taddr + 192), "r"(taddr + 224));
 #pragma unroll
   for (int i = 0; i < 8; ++i) v[i] = make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
 }
