@@ -2,10 +2,11 @@
 // the float pyramid, maps, ReLU states and gradients of n equally sized
 // images, and the launch sequences of the forward and backward.
 //
-// Nothing of the responses survives the forward: the backward recomputes each
-// tile's spectrum and e + i o.  The per-cell scratch (complex cells C and
-// their gradient) exists for a chunk of images at a time; the forward and the backward walk the chunks in order, and the
-// entries of images in different chunks share the same scratch.
+// The forward's e + i o and tile spectra are kept for the backward where there
+// is memory for them (reserve_kept); otherwise the backward recomputes them.
+// The per-cell scratch (complex cells C and their gradient) exists for a chunk
+// of images at a time; the forward and the backward walk the chunks in order,
+// and the entries of images in different chunks share the same scratch.
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -292,8 +292,9 @@ __device__ __forceinline__ int perm128d(int k) { return 8 * (k & 15) + (k >> 4);
 // spectrum into TMEM, Hermitian half into this CTA's slot of `xscratch`) and z
 // per orientation by the forward's inverse passes (G read from L2 instead of
 // staged).  That costs 60 k + 30 k cycles per item + orientation against 40 k +
-// 22 k here and 12 bytes of memory an output: 16 images of 512 x 512 took 1680
-// us recomputed and take 1165 kept, the forward 864 us instead of 791.
+// 21 k here, which take 8 bytes more memory an output and orientation: 16
+// images of 512 x 512 take 1640 us recomputed and 1130 kept, the forward 864 us
+// instead of 791.
 //
 // The x-passes of both directions run on the same rows, so a warp takes
 // blocks of four valid rows through all of them (inverse 8 and 16, magnitude,

@@ -538,7 +538,8 @@ struct Engine {
         // the first launch also zeroes the per-detection reset words
         for (size_t l = 0; l < pyrFirst.size(); ++l)
           launch_pyr(d_pyr + pyrFirst[l], pyrCount[l], pyrLevels[l], pyrMaxW[l], pyrMaxH[l], s,
-                     l == 0 ? d_maxKeys : nullptr, l == 0 ? static_cast<int>(resetBytes / sizeof(unsigned int)) : 0);
+                     l == 0 ? d_maxKeys : nullptr, l == 0 ? static_cast<int>(resetBytes / sizeof(unsigned int)) : 0,
+                     pdl_enabled());
         break;
       // stages 1-3 follow the previous stage's kernel with programmatic
       // dependent launch (each waits in the kernel for its predecessor)

@@ -1361,13 +1361,13 @@ __global__ void k_set_out(KpOut* __restrict__ d, KpOut v) { *d = v; }
 void launch_set_out(KpOut* d, const KpOut& v, cudaStream_t s) { k_set_out<<<1, 1, 0, s>>>(d, v); }
 
 void launch_pyr(const PyrJob* d_jobs, int njobs, int levels, int maxW, int maxH, cudaStream_t s,
-                unsigned int* reset, int resetWords) {
+                unsigned int* reset, int resetWords, bool pdl) {
   if (njobs <= 0 || levels <= 0) return;
   const int T = 32 >> (levels - 1);
   dim3 g((maxW + T - 1) / T, (maxH + T - 1) / T, njobs);
   auto k = levels == 3 ? k_pyr_down<3> : levels == 2 ? k_pyr_down<2> : k_pyr_down<1>;
   // the launches after the first (the one with the reset) wait in the kernel
-  launch_ex(k, g, kPyrThreads, 0, s, !reset, d_jobs, reset, resetWords);
+  launch_ex(k, g, kPyrThreads, 0, s, pdl && !reset, d_jobs, reset, resetWords);
 }
 void launch_gabor(const ScaleDev* d_sd, const TileWork* d_work, int nwork, int grid, unsigned int* d_fault,
                   cudaStream_t s, bool pipelined, bool pdl) {

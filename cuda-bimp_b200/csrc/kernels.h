@@ -50,9 +50,11 @@ size_t stencil_smem_bytes();
 // deepest-level size over the jobs
 void launch_set_out(KpOut* d, const KpOut& v, cudaStream_t s);
 // reset/resetWords: words the launch's first CTA zeroes before anything else
-// of the detection runs (the map maxima and the fault word), or null.
+// of the detection runs (the map maxima and the fault word); null for the
+// launches after the first, which wait for the one before in the kernel (pdl: they
+// overlap its end).
 void launch_pyr(const PyrJob* d_jobs, int njobs, int levels, int maxW, int maxH, cudaStream_t s,
-                unsigned int* reset = nullptr, int resetWords = 0);
+                unsigned int* reset = nullptr, int resetWords = 0, bool pdl = false);
 // d_fault: word that receives 1 if a bounded device wait expired.
 // pipelined: the warp-specialised variant (k_gabor_tiles_ws), for work whose
 // scales all have V <= pipelined_tile_max_valid(); otherwise the phased one

@@ -26,7 +26,9 @@ constexpr TileCost kForwardCost = {1.4, 0.481, 0.0741};
 constexpr TileCost kBackwardCost = {1.97, 0.62, 0.0543};
 // Backward from kept responses (between that case, 40.8 k, 13.4 k, 1.30 k, and
 // 1333 x 1001, 35.9 k, 15.3 k, 1.08 k of 22.5 k cycles; residual 10 k of about
-// 210 k).
+// 210 k).  The y-passes through tensor memory made an orientation 1.4 k cycles
+// shorter; weights refitted to that moved the two cases' backward by +1.2% and
+// -0.4%, so these stayed.
 constexpr TileCost kBackwardKeptCost = {1.75, 0.62, 0.0535};
 
 // Balanced plan for a persistent grid of `grid` CTAs.  The (tile,
