@@ -634,9 +634,9 @@ def uhd_adjoint(frames, dev, stream) -> dict:
            "train_step_mpixel_s": round(n * 3840 * 2160 / ((f_ms + b_ms) * 1e-3) / 1e6, 1),
            "device_bytes_arena": adj.device_bytes(), "device_bytes_held": int(held),
            "note": "peak device memory held by the adjoint (its arena plus the gradient output), measured "
-                   "as the drop in free device memory; the backward recomputes each tile's spectrum and "
-                   "e + i o (nothing of the forward's responses is stored); complex cells, their gradient "
-                   "and the inhibition maps exist for a chunk of frames at a time"}
+                   "as the drop in free device memory; this many frames are past the size up to which "
+                   "the forward keeps e + i o and the tile spectra, so the backward recomputes them; complex "
+                   "cells and their gradient exist for a chunk of frames at a time"}
     adj.close()
     del x, masks, grad
     torch.cuda.synchronize()
