@@ -193,6 +193,7 @@ __device__ __forceinline__ int widx(int y, int p) { return y * kWPitch + 9 * (p 
 // spectrum.
 struct PadLayout {
   static constexpr int kHalf = 64 * kWPitch;
+  static constexpr bool kFewRegs = false;
   static __device__ __forceinline__ int at(int y, int p) { return widx(y, p); }
   // lanes 16 j + i: columns of group j (i < 8) and of group j + 8
   static __device__ __forceinline__ int col(int lane) { return 8 * ((lane >> 4) + 8 * ((lane >> 3) & 1)) + (lane & 7); }
@@ -201,6 +202,7 @@ struct PadLayout {
 // rotate inside each group of eight, odd rows swap the halves of each 16.
 struct RotLayout {
   static constexpr int kHalf = 64 * kTile;
+  static constexpr bool kFewRegs = true;   // (its loop over the orientations keeps more of them)
   static __device__ __forceinline__ int at(int y, int p) { return y * kTile + (phys(p) ^ ((y & 1) << 3)); }
   static __device__ __forceinline__ int col(int lane) { return lane; }
 };
@@ -376,7 +378,7 @@ __device__ __forceinline__ void raw_window_copy(const ScaleDev* sd, int R0, int 
     any[k] = __any_sync(0xffffffffu, mine[k]);
     c[k] = any[k] ? window_src(C0 - kX, i, sd->fftW, sd->dataW, kX) : 0;
   }
-  constexpr int kBatch = FLT ? 4 : 8;   // rows whose loads are in flight together (registers)
+  constexpr int kBatch = 4;   // rows whose loads are in flight together (eight: spills in the pipelined kernel)
 #pragma unroll 1
   for (int i0 = 0; i0 < 8; i0 += kBatch) {
     T v[kBatch][4];
@@ -483,7 +485,7 @@ __device__ __forceinline__ void tile_forward_spectrum(const typename RawWindow<F
     const float sign = hc.conj ? -1.f : 1.f;
     const float2* src = hc.slot == 64 ? Nyq : Xh + hc.slot;
     const int st = hc.slot == 64 ? 1 : 64;
-#pragma unroll(SAVE_X ? 1 : 4)
+#pragma unroll(SAVE_X || LY::kFewRegs ? 1 : 4)
     for (int q = 0; q < 4; ++q) {
       const int k2 = h + 4 * q;
       const int kb = hc.conj ? (16 - k2) & 15 : k2;
@@ -843,7 +845,11 @@ k_gabor_tiles(const ScaleDev* __restrict__ sds, const TileWork* __restrict__ wor
 // named barriers hand them over (full: Y -> X, empty: X -> Y), and each group
 // orders its own passes with a 256-thread named barrier, so no CTA-wide
 // barrier stands inside the orientation loop.  G_o is read from L2 (the
-// space of the TMA ring holds the second buffer).  Needs V <= kWsRows.
+// second buffer takes the space it would be staged in), a thread's eight values
+// as two 16-byte loads.  Needs V <= kWsRows.  64 mixed images, one CTA a tile:
+// 7.62 ms a detection (8.69 with the values loaded one by one in the order of
+// the stored spectrum and the window staged value by value; k_gabor_tiles
+// 6.90).
 constexpr int kWsRows = 104;                                  // largest V this kernel takes
 constexpr int kWsBuf = kWsRows * kTile;                       // complex per row buffer
 constexpr int kWsSmemW = 2 * kWsBuf * 8;                      // both row buffers (also the forward scratch)
@@ -896,7 +902,11 @@ k_gabor_tiles_ws(const ScaleDev* __restrict__ sds, const TileWork* __restrict__ 
     const int R0 = ty * V, C0 = tx * V;
     __syncthreads();   // previous tile finished with every buffer
     auto* raw = reinterpret_cast<typename RawWindow<FLT>::T*>(Wb + RotLayout::kHalf);
-    raw_window_copy<FLT>(sd, R0, C0, raw, 0, 0, t);
+    raw_chunks_load<FLT>(sd, R0, C0, raw, t);
+    raw += (C0 - kX) & (WindowSpan<FLT>::kVals - 1);
+    const WindowSpan<FLT> span(sd, C0);
+    if (!span.all()) raw_window_copy<FLT>(sd, R0, C0, raw, span.iA, span.iB, t);
+    cp_async_wait();
     __syncthreads();
     tile_forward_spectrum<FLT, false, RotLayout>(raw, Wb, Nyq, tw, tlane, nullptr, t, [] {});
     tmem_fence_before();
@@ -906,32 +916,30 @@ k_gabor_tiles_ws(const ScaleDev* __restrict__ sds, const TileWork* __restrict__ 
       for (int o = oB; o < oE; ++o) {
         const int b = (o - oB) & 1;
         float2* Wo = Wb + b * kWsBuf;
-        const float* __restrict__ Go = sd->G + (size_t)o * kSpecFloats;
+        const float4* __restrict__ Go = reinterpret_cast<const float4*>(sd->G + (size_t)o * kSpecFloats) + glane(pI1);
         // I1: y-dim pass B' with the spectrum product (TMEM in, TMEM y-area
-        // out); each quarter's G values are loaded one quarter ahead
-        float g[8];
-#pragma unroll
-        for (int k1 = 0; k1 < 8; ++k1) g[k1] = __ldg(Go + gpos(8 * hY + k1, glane(pI1)));
+        // out); each quarter's G values, two 16-byte loads, come one quarter
+        // ahead
+        float4 ga = __ldg(Go + 2 * hY * kTile), gb = __ldg(Go + (2 * hY + 1) * kTile);
 #pragma unroll 1
         for (int q = 0; q < 8; ++q) {
           const int k2 = hY + 2 * q;
           float2 v[8];
-          float gn[8];
           const int k2n = q < 7 ? k2 + 2 : k2;
-#pragma unroll
-          for (int k1 = 0; k1 < 8; ++k1) gn[k1] = __ldg(Go + gpos(8 * k2n + k1, glane(pI1)));
+          const float4 gan = __ldg(Go + 2 * k2n * kTile), gbn = __ldg(Go + (2 * k2n + 1) * kTile);
           tmem_load8(tlane + 16 * k2, v);
           float2 twr[8];
 #pragma unroll
           for (int n1 = 1; n1 < 8; ++n1) twr[n1] = tw[n1 * 17 + k2];
+          const float g[8] = {ga.x, ga.y, ga.z, ga.w, gb.x, gb.y, gb.z, gb.w};
 #pragma unroll
           for (int k1 = 0; k1 < 8; ++k1) v[k1] = c_scale(v[k1], g[k1]);
           dft8<true>(v);
 #pragma unroll
           for (int n1 = 0; n1 < 8; ++n1)
             tmem_store1(tlane + kTmemY + 2 * (16 * n1 + k2), n1 ? c_mulc(v[n1], twr[n1]) : v[0]);
-#pragma unroll
-          for (int k1 = 0; k1 < 8; ++k1) g[k1] = gn[k1];
+          ga = gan;
+          gb = gbn;
         }
         tmem_wait_st();
         tmem_fence_before();
