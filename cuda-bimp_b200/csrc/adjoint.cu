@@ -281,11 +281,16 @@ struct bimp_adjoint {
     std::vector<size_t> offZ, offX;   // per entry, in `keep`
     if (!pipelined) reserve_kept(sds, offZ, offX);
     std::vector<TileWork> plans;
+    // CTAs of the plans: one per SM (BIMP_ADJOINT_GRID overrides it, for tests:
+    // on a few CTAs small images too make items of several orientations and
+    // CTAs of several items)
+    int ctas = num_sms();
+    if (const char* g = std::getenv("BIMP_ADJOINT_GRID")) ctas = std::max(1, std::atoi(g));
     for (int i0 = 0; i0 < n; i0 += chunk) {
       const std::vector<TileWork> part(tiles.begin() + tileStart[i0], tiles.begin() + tileStart[std::min(n, i0 + chunk)]);
       auto add = [&](std::vector<Plan>& to, const TileCost& cost) {
         Plan p;
-        const std::vector<TileWork> work = split_plan(part, sds, cost, num_sms(), &p.grid);
+        const std::vector<TileWork> work = split_plan(part, sds, cost, ctas, &p.grid);
         p.first = plans.size();
         p.items = static_cast<int>(work.size());
         plans.insert(plans.end(), work.begin(), work.end());
