@@ -119,6 +119,8 @@ _PROTOS = [
                                            C.POINTER(C.c_size_t), C.POINTER(C.c_size_t)]),
     ("bimp_adjoint_forward", C.c_int, [C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p, C.c_void_p, C.c_void_p]),
     ("bimp_adjoint_backward", C.c_int, [C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p, C.c_void_p]),
+    ("bimp_adjoint_status", C.c_int, [C.c_void_p, C.c_void_p]),
+    ("bimp_adjoint_inject_fault", C.c_int, [C.c_void_p, C.c_void_p]),
     ("bimp_adjoint_dense_map", C.c_int, [C.c_void_p, C.c_int, C.c_int, C.c_void_p, C.c_size_t, C.c_void_p]),
     ("bimp_adjoint_complex_map", C.c_int, [C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_size_t,
                                            C.c_void_p]),

@@ -611,6 +611,12 @@ class Adjoint:
                 "adjoint_backward")
         return grad, self._gp
 
+    def check(self, stream=None):
+        """Waits for the stream; raises if a bounded device wait expired in a
+        forward or backward since the last check (bimp_adjoint_status): those
+        two return before their kernels run."""
+        L.check(L.lib().bimp_adjoint_status(self._h, _stream_ptr(stream)), "adjoint")
+
     def dense_map(self, image: int, scale: int):
         torch = _torch()
         off, w, h = self.layout[scale]

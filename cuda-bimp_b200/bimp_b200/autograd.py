@@ -48,6 +48,7 @@ class SummedKeypointMapLoss(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad_out):
         g, gp = ctx.adj.backward()
+        ctx.adj.check()   # an expired device wait raises here
         go = grad_out.to(torch.float64)
         return (g * go.to(g.dtype)).clone(), (gp * go).to(ctx.theta_dtype), None, None
 

@@ -106,7 +106,8 @@ struct bimp_adjoint {
   std::vector<int> tileStart, stenStart, stenBStart;   // per image (n + 1 entries)
   double* d_loss = nullptr;               // [0] loss, [1..4] parameter gradients
   double* d_gp = nullptr;
-  unsigned int* d_max = nullptr;          // per entry + fault word
+  unsigned int* d_max = nullptr;          // per entry, then the fault word
+  unsigned int* d_fault = nullptr;        // bits set by the kernels when a bounded wait expired, until status() reads them
 
   // Memory for the forward's e + i o and tile spectra, which let the backward
   // start from them instead of transforming every tile again.  It is taken
@@ -337,6 +338,8 @@ struct bimp_adjoint {
     d_glvl = glvl[0];
     d_M = reinterpret_cast<float*>(b + offM);
     d_max = reinterpret_cast<unsigned int*>(b + offMax);
+    d_fault = d_max + sds.size();
+    ADJ_CUDA(cudaMemset(d_fault, 0, sizeof(unsigned int)));
     for (size_t e2 = 0; e2 < sds.size(); ++e2) {
       ScaleDev& d = sds[e2];
       const int i = d.image, si = static_cast<int>(e2 % nScales);
@@ -408,21 +411,31 @@ struct bimp_adjoint {
     return BIMP_OK;
   }
 
+  // What stream s has run: reports an expired wait once.
+  int status(cudaStream_t s) {
+    unsigned int fault = 0;
+    ADJ_CUDA(cudaMemcpyAsync(&fault, d_fault, sizeof(fault), cudaMemcpyDeviceToHost, s));
+    ADJ_CUDA(cudaStreamSynchronize(s));
+    if (!fault) return BIMP_OK;
+    ADJ_CUDA(cudaMemsetAsync(d_fault, 0, sizeof(fault), s));
+    ADJ_CUDA(cudaStreamSynchronize(s));
+    return afail(BIMP_ERR_CUDA, "a bounded device wait expired in a forward or backward: its results are not valid");
+  }
+
   int forward(const float* imgs, size_t pitch, const float* masks, double* loss, cudaStream_t s) {
     // the n images as one block of n * H rows
     ADJ_CUDA(cudaMemcpy2DAsync(d_lvl0, sizeof(float) * lp[0], imgs, sizeof(float) * pitch, sizeof(float) * W,
                                (size_t)n * H, cudaMemcpyDeviceToDevice, s));
     ADJ_CUDA(cudaMemcpyAsync(d_M, masks, sizeof(float) * maskStride * n, cudaMemcpyDeviceToDevice, s));
     for (int l = 1; l <= maxLevel; ++l) launch_pyr_f(d_pyr + (l - 1) * n, n, lw[l], lh[l], s);
-    ADJ_CUDA(cudaMemsetAsync(d_max, 0, sizeof(unsigned int) * (h_sd.size() + 1), s));
+    ADJ_CUDA(cudaMemsetAsync(d_max, 0, sizeof(unsigned int) * h_sd.size(), s));
     ADJ_CUDA(cudaMemsetAsync(d_loss, 0, sizeof(double) * 5, s));
-    unsigned int* fault = d_max + h_sd.size();
     for (int i0 = 0; i0 < n; i0 += chunk) {
       const int i1 = std::min(n, i0 + chunk);
       const Plan& p = fwdPlan[i0 / chunk];
-      launch_gabor_flt(d_sd, d_tiles + p.first, p.items, p.grid, fault, s, pipelined, keep != nullptr);
-      launch_stencil(d_sd, d_sten + stenStart[i0], stenStart[i1] - stenStart[i0], fault, s, kStencilAdj, false, d_loss,
-                     d_gp);
+      launch_gabor_flt(d_sd, d_tiles + p.first, p.items, p.grid, d_fault, s, pipelined, keep != nullptr);
+      launch_stencil(d_sd, d_sten + stenStart[i0], stenStart[i1] - stenStart[i0], d_fault, s, kStencilAdj, false,
+                     d_loss, d_gp);
     }
     if (loss) ADJ_CUDA(cudaMemcpyAsync(loss, d_loss, sizeof(double), cudaMemcpyDeviceToDevice, s));
     ADJ_CUDA(cudaGetLastError());
@@ -438,7 +451,7 @@ struct bimp_adjoint {
       const int i1 = std::min(n, i0 + chunk);
       launch_stencil_bwd(d_sd, d_stenB + stenBStart[i0], stenBStart[i1] - stenBStart[i0], s);
       const Plan& p = bwdPlan[i0 / chunk];
-      launch_gabor_bwd(d_sd, d_tiles + p.first, p.items, p.grid, d_xscr, d_gp, s, keep != nullptr);
+      launch_gabor_bwd(d_sd, d_tiles + p.first, p.items, p.grid, d_xscr, d_gp, d_fault, s, keep != nullptr);
     }
     for (int l = maxLevel; l >= 1; --l) launch_pyr_f_adj(d_pyrAdj + (l - 1) * n, n, lw[l - 1], lh[l - 1], s);
     ADJ_CUDA(cudaMemcpy2DAsync(grad, sizeof(float) * pitch, d_glvl, sizeof(float) * lp[0], sizeof(float) * W,
@@ -511,6 +524,19 @@ int bimp_adjoint_backward(bimp_adjoint* a, float* d_grad, size_t pitch, double* 
   if (!a || !d_grad || pitch < (size_t)a->W) return afail(BIMP_ERR_INVALID, "bad backward arguments");
   ADJ_CUDA(cudaSetDevice(a->device));
   return a->backward(d_grad, pitch, d_grad_params, static_cast<cudaStream_t>(stream));
+}
+
+int bimp_adjoint_status(bimp_adjoint* a, void* stream) {
+  if (!a) return afail(BIMP_ERR_INVALID, "adjoint is null");
+  ADJ_CUDA(cudaSetDevice(a->device));
+  return a->status(static_cast<cudaStream_t>(stream));
+}
+
+int bimp_adjoint_inject_fault(bimp_adjoint* a, void* stream) {
+  if (!a) return afail(BIMP_ERR_INVALID, "adjoint is null");
+  ADJ_CUDA(cudaSetDevice(a->device));
+  ADJ_CUDA(cudaMemsetAsync(a->d_fault, 1, sizeof(unsigned int), static_cast<cudaStream_t>(stream)));
+  return BIMP_OK;
 }
 
 int bimp_adjoint_dense_map(bimp_adjoint* a, int image, int scale, float* d_out, size_t ld, void* stream) {

@@ -332,7 +332,7 @@ struct BwEntries {
 template <bool KEPT>
 __global__ void __launch_bounds__(kTileThreads, 1)
 k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__ work, int nwork,
-                  float2* __restrict__ xscratch, double* __restrict__ gparams) {
+                  float2* __restrict__ xscratch, double* __restrict__ gparams, unsigned int* __restrict__ fault_word) {
   extern __shared__ float4 smem4b[];
   char* base = reinterpret_cast<char*>(smem4b);
   float2* W = reinterpret_cast<float2*>(base);
@@ -363,6 +363,7 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
   const int h = t >> 7, pcol = PadLayout::col(t & 127);   // row group, this lane's column
   const int warp = t >> 5, quad = warp & 3, lane = t & 31;
   uint32_t phW = 0;
+  bool fault = false;   // a wait of this thread expired: what follows is not valid
   double accA = 0.0, accR = 0.0;
   for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
     const TileWork item = work[w];
@@ -468,7 +469,7 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
         named_barrier(1 + quad, kTileThreads / 4);   // the lane block's first y-pass is complete
         tmem_fence_after();
         if (o > oB) {   // every warp is done with the previous orientation's accumulation
-          mbar_wait(barW, phW);
+          if (!mbar_wait(barW, phW)) fault = true;
           phW ^= 1u;
           __syncwarp();
         }
@@ -494,7 +495,7 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
       // orientation's accumulation
       auto wait_w = [&] {
         if (KEPT && o > oB) {
-          mbar_wait(barW, phW);
+          if (!mbar_wait(barW, phW)) fault = true;
           phW ^= 1u;
           __syncwarp();
         }
@@ -823,6 +824,7 @@ k_gabor_tiles_bwd(const ScaleDev* __restrict__ sds, const TileWork* __restrict__
   __syncthreads();
   tmem_fence_after();
   if ((t >> 5) == 0) tmem_dealloc_warp(*tmemSlot);
+  if (fault) atomicOr(fault_word, 4u);
   block_add_double(accA, gparams + 0);
   block_add_double(accR, gparams + 1);
 }

@@ -34,8 +34,8 @@
 // of the forward transform and staged windows (241.2), x-passes without CTA
 // barriers (238.0), balanced first y-passes (232.1) and, in larger batches of
 // work, the plan's refitted costs.  Every mbarrier wait is bounded; on expiry
-// the kernel records a fault in *fault, waits once more (bounded) for its copies
-// and carries on, and the host reports the fault.
+// the thread that saw it sets a bit of *fault_word, the kernel waits once more
+// (bounded) for its copies and carries on, and the host reports the fault.
 //
 // Included inside namespace bimp_b200 by kernels.cu, after the helpers it uses
 // (pad_src, pmod, c_w128).
@@ -251,7 +251,7 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
                : "memory");
 }
 // Bounded wait for phase `parity` of `bar`; false if it did not complete.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
+[[nodiscard]] __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   for (int i = 0; i < (1 << 22); ++i) {
     uint32_t done;
     asm volatile(
@@ -821,10 +821,12 @@ k_gabor_tiles(const ScaleDev* __restrict__ sds, const TileWork* __restrict__ wor
     }
   }
   if (fault) {
-    // a wait expired: record it, then give the copies still in flight a
-    // second bounded chance to land before the CTA releases its memory
-    if (t == 0) atomicOr(fault_word, 1u);
-    mbar_wait(bar0, ph ^ 1);
+    // a wait expired: the thread that saw it records it (warps come to a wait
+    // at different times: none speaks for another), then the copies still in
+    // flight get a second bounded chance to land before the CTA releases its
+    // memory
+    atomicOr(fault_word, 1u);
+    (void)mbar_wait(bar0, ph ^ 1);
   }
   tmem_fence_before();
   __syncthreads();

@@ -672,7 +672,7 @@ k_stencil(const ScaleDev* __restrict__ sds, const int2* __restrict__ work, int n
     // before the CTA can end, the last copy into each buffer must land
     if (lane == 0) {
       for (int k = issued - 1; k >= 0 && k >= issued - kStBufs; --k)
-        mbar_wait(full0 + 8 * (k % kStBufs), (k / kStBufs) & 1);
+        (void)mbar_wait(full0 + 8 * (k % kStBufs), (k / kStBufs) & 1);
     }
     return;
   }
@@ -1410,9 +1410,9 @@ void launch_stencil_bwd(const ScaleDev* d_sd, const int2* d_work, int nwork, cud
 }
 
 void launch_gabor_bwd(const ScaleDev* d_sd, const TileWork* d_work, int nwork, int grid, float2* d_xscratch,
-                      double* d_gparams, cudaStream_t s, bool kept) {
+                      double* d_gparams, unsigned int* d_fault, cudaStream_t s, bool kept) {
   auto k = kept ? k_gabor_tiles_bwd<true> : k_gabor_tiles_bwd<false>;
-  if (nwork > 0) k<<<grid, kTileThreads, kGaborBwdSmem, s>>>(d_sd, d_work, nwork, d_xscratch, d_gparams);
+  if (nwork > 0) k<<<grid, kTileThreads, kGaborBwdSmem, s>>>(d_sd, d_work, nwork, d_xscratch, d_gparams, d_fault);
 }
 void launch_stencil(const ScaleDev* d_sd, const int2* d_work, int nwork, unsigned int* d_fault, cudaStream_t s,
                     int mode, bool pdl, double* d_loss, double* d_gparams) {

@@ -55,7 +55,8 @@ void launch_set_out(KpOut* d, const KpOut& v, cudaStream_t s);
 // overlap its end).
 void launch_pyr(const PyrJob* d_jobs, int njobs, int levels, int maxW, int maxH, cudaStream_t s,
                 unsigned int* reset = nullptr, int resetWords = 0, bool pdl = false);
-// d_fault: word that receives 1 if a bounded device wait expired.
+// d_fault: word that gets a bit set if a bounded device wait expired (1: tile
+// kernel, 2: stencil, 4: tile backward).
 // pipelined: the warp-specialised variant (k_gabor_tiles_ws), for work whose
 // scales all have V <= pipelined_tile_max_valid(); otherwise the phased one
 // pdl: launched with programmatic stream serialisation after the previous
@@ -116,6 +117,6 @@ void launch_stencil_bwd(const ScaleDev* d_sd, const int2* d_work, int nwork, cud
 // CTAs; to recompute, d_xscratch holds grid x kSpecHalf float2 (one tile
 // spectrum per CTA)
 void launch_gabor_bwd(const ScaleDev* d_sd, const TileWork* d_work, int nwork, int grid, float2* d_xscratch,
-                      double* d_gparams, cudaStream_t s, bool kept);
+                      double* d_gparams, unsigned int* d_fault, cudaStream_t s, bool kept);
 
 }  // namespace bimp_b200

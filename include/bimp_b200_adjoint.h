@@ -57,6 +57,16 @@ int bimp_adjoint_forward(bimp_adjoint* a, const float* d_images, size_t pitch, c
  * images) and dL/d(alpha, rho, w_tan, w_rad) into 4 device doubles. */
 int bimp_adjoint_backward(bimp_adjoint* a, float* d_grad, size_t pitch, double* d_grad_params, void* stream);
 
+/* Waits for `stream` and returns BIMP_ERR_CUDA, once, if a bounded device wait
+ * expired in a forward or backward since the last report: the results written
+ * since then are not valid.  (forward and backward return before their kernels
+ * run and so cannot say it.) */
+int bimp_adjoint_status(bimp_adjoint* a, void* stream);
+
+/* Marks an expired wait as the kernels do, in stream order, so that a program
+ * can test what it does about one. */
+int bimp_adjoint_inject_fault(bimp_adjoint* a, void* stream);
+
 /* Summed keypoint map of image i, scale s of the last forward (device copy,
  * data_h x data_w, row pitch ld floats). */
 int bimp_adjoint_dense_map(bimp_adjoint* a, int image, int scale, float* d_out, size_t ld, void* stream);
