@@ -136,6 +136,7 @@ _PROTOS = [
                                       C.c_int, C.POINTER(C.c_int)]),
     ("bimp_batch_counts", C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p]),
     ("bimp_batch_count", C.c_int, [C.c_void_p, C.c_int, C.POINTER(C.c_int), C.c_void_p]),
+    ("bimp_batch_inject_fault", C.c_int, [C.c_void_p, C.c_void_p]),
     ("bimp_batch_keypoints_device", C.c_int, [C.c_void_p, C.c_int, C.POINTER(C.c_void_p),
                                               C.POINTER(C.c_size_t)]),
     ("bimp_batch_scale_info", C.c_int, [C.c_void_p, C.c_int, C.c_int, C.POINTER(ScaleInfo)]),

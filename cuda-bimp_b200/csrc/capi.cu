@@ -1187,9 +1187,18 @@ int bimp_batch_count(bimp_batch* b, int i, int* n_found, void* stream) {
   if (!b || !n_found || i < 0 || i >= b->eng.nImages) return fail(BIMP_ERR_INVALID, "bad batch count arguments");
   BIMP_CUDA(cudaSetDevice(b->eng.device));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  BIMP_CUDA(cudaMemcpyAsync(b->h_totals + 1 + i, b->eng.d_totals + i, sizeof(int), cudaMemcpyDeviceToHost, s));
+  // the fault word and the totals up to image i's lie side by side: one copy
+  BIMP_CUDA(cudaMemcpyAsync(b->h_totals, b->eng.d_fault, sizeof(int) * (2 + (size_t)i), cudaMemcpyDeviceToHost, s));
   BIMP_CUDA(cudaStreamSynchronize(s));
+  if (b->h_totals[0]) return fail(BIMP_ERR_CUDA, "a bounded device wait expired");
   *n_found = b->h_totals[1 + i];
+  return BIMP_OK;
+}
+
+int bimp_batch_inject_fault(bimp_batch* b, void* stream) {
+  if (!b) return fail(BIMP_ERR_INVALID, "batch is null");
+  BIMP_CUDA(cudaSetDevice(b->eng.device));
+  BIMP_CUDA(cudaMemsetAsync(b->eng.d_fault, 1, sizeof(unsigned int), static_cast<cudaStream_t>(stream)));
   return BIMP_OK;
 }
 

@@ -81,8 +81,13 @@ int bimp_batch_run(bimp_batch* batch, void* stream);
 /* Copies the per-image keypoint totals (n_images ints) to device memory. */
 int bimp_batch_counts(bimp_batch* batch, int* d_counts, void* stream);
 
-/* Keypoint total of image i to host memory; waits for `stream`. */
+/* Keypoint total of image i to host memory; waits for `stream`.  BIMP_ERR_CUDA
+ * if a bounded device wait expired in the last run. */
 int bimp_batch_count(bimp_batch* batch, int i, int* n_found, void* stream);
+
+/* Marks an expired wait as the kernels do, in stream order and until the next
+ * run, so that a program can test what it does about one. */
+int bimp_batch_inject_fault(bimp_batch* batch, void* stream);
 
 /* Internal 7 x ld keypoint matrix of image i, (scale, y, x) order; only the
  * first min(count, ld) columns are written. */
