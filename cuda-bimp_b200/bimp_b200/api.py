@@ -475,14 +475,18 @@ class Batch:
             pitch = C.c_size_t()
             L.check(L.lib().bimp_batch_image(h, i, C.byref(ptr), C.byref(pitch)), "batch_image")
             self._inputs.append((ptr.value, pitch.value))
-        # aliases of the library's input and keypoint buffers, made once
-        self._input_tensors = [_wrap_device(p, (hh, w), (pitch, 1), "|u1")
-                               for (p, pitch), (w, hh) in zip(self._inputs, self.sizes)]
-        self._kp = []
-        for i in range(n):
-            ptr, ld = C.c_void_p(), C.c_size_t()
-            L.check(L.lib().bimp_batch_keypoints_device(h, i, C.byref(ptr), C.byref(ld)), "batch_keypoints")
-            self._kp.append(_wrap_device(ptr.value, (KP_VECTOR_LENGTH, ld.value), (4 * ld.value, 4), "<f4"))
+        # aliases of the library's input and keypoint buffers, made once; what is
+        # handed out is their .data, which shares the memory but no autograd state
+        # (an in-place operation on one view must not mark the next call's), and
+        # they are ordinary tensors also where the batch is made in inference mode
+        with torch.inference_mode(False):
+            self._input_tensors = [_wrap_device(p, (hh, w), (pitch, 1), "|u1")
+                                   for (p, pitch), (w, hh) in zip(self._inputs, self.sizes)]
+            self._kp = []
+            for i in range(n):
+                ptr, ld = C.c_void_p(), C.c_size_t()
+                L.check(L.lib().bimp_batch_keypoints_device(h, i, C.byref(ptr), C.byref(ld)), "batch_keypoints")
+                self._kp.append(_wrap_device(ptr.value, (KP_VECTOR_LENGTH, ld.value), (4 * ld.value, 4), "<f4"))
         self._counts = torch.zeros(n, dtype=torch.int32, device="cuda")
 
     def input_view(self, i: int):
@@ -491,7 +495,7 @@ class Batch:
 
     def input_tensor(self, i: int):
         """uint8 CUDA tensor (h x w, row stride = pitch) aliasing image i's input."""
-        return self._input_tensors[i]
+        return self._input_tensors[i].data
 
     def load(self, images, stream=None):
         """Copy uint8 images (numpy or CUDA tensors) into the batch inputs."""
@@ -548,7 +552,7 @@ class Batch:
         columns as the last run found (waits for it)."""
         n = C.c_int(0)
         L.check(L.lib().bimp_batch_count(self._h, int(i), C.byref(n), _stream_ptr()), "batch_keypoints")
-        return self._kp[i][:, :min(n.value, self.kp_capacity)]
+        return self._kp[i].data[:, :min(n.value, self.kp_capacity)]
 
     def close(self):
         if getattr(self, "_h", None) is not None:
