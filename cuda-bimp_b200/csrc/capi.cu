@@ -408,11 +408,13 @@ struct Engine {
     stenStart.push_back(nSten);
     nRows = static_cast<int>(rows.size());
     const size_t offSd = a.reserve(sizeof(ScaleDev) * sds.size());
-    {   // the tile buffer holds the largest plan the autotuner may choose
-      // (and room for other grids a caller may ask for: a split plan's
-      // padded list holds about nTiles + 3 grid entries when the tiles'
-      // costs are within a factor of two; a plan beyond the buffer is
-      // refused by retile)
+    {   // the tile buffer holds twice the largest plan the autotuner may choose
+      // and twice the room of a grid below it: a split plan's padded list is
+      // its CTAs times the most items of one, so that a list of one item a CTA
+      // becomes one of two with a small change of the cost model's weights.
+      // (Over random batches and grids up to 4000, what the weights of an
+      // earlier kernel accepted with a buffer of half this size, these accept
+      // too; a plan beyond the buffer is refused by retile.)
       tileCap = nWork;
       int maxTiles = 0;
       const int grids[4] = {0, sms, 2 * sms, defGrid};
@@ -424,7 +426,7 @@ struct Engine {
             tileCap = std::max(tileCap, static_cast<int>(work_list(tmp, policy, order, g, &nt, &ng).size()));
             maxTiles = std::max(maxTiles, nt);
           }
-      tileCap = std::max(tileCap, 2 * maxTiles + 6 * sms);
+      tileCap = 2 * std::max(tileCap, 2 * maxTiles + 6 * sms);
     }
     const size_t offTiles = a.reserve(sizeof(TileWork) * std::max<size_t>(1, (size_t)tileCap));
     const size_t offSten = a.reserve(sizeof(int2) * std::max<size_t>(1, sten.size()));
