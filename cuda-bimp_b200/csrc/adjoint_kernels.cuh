@@ -57,10 +57,22 @@ __global__ void __launch_bounds__(256) k_pyr_down_f(const PyrJobF* __restrict__ 
 // positions: weight w[k] with which source position p enters output Y0 + k (the
 // outputs past the ends get weight 0).  Position p itself, and next to a border
 // the window position -1, -2, n or n + 1 that reflects onto it, which lies in
-// the window of the same three outputs (n >= 5).
+// the window of the same three outputs.  Below 5 positions, where a window
+// position can reflect twice, there are two outputs at most: their taps are
+// reflected one by one.
 __device__ __forceinline__ int pyr_adj_weights(int p, int n, float (&w)[3]) {
-  const int Y0 = (p - 1) >> 1, m = (n + 1) >> 1;
   auto f = [](int d) { return d == 0 ? 6.f : d == 1 || d == -1 ? 4.f : d == 2 || d == -2 ? 1.f : 0.f; };
+  const int m = (n + 1) >> 1;
+  if (n < 5) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      w[k] = 0.f;
+      for (int i = -2; i <= 2; ++i)
+        if (k < m && reflect101(2 * k + i, n) == p) w[k] += f(i);
+    }
+    return 0;
+  }
+  const int Y0 = (p - 1) >> 1;
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     const int Y = Y0 + k;
@@ -74,62 +86,46 @@ __device__ __forceinline__ int pyr_adj_weights(int p, int n, float (&w)[3]) {
 
 // g_src(r101(2y+i), r101(2x+j)) += w_i w_j / 256 * g_dst(y, x), gathered: a
 // thread adds what reaches four adjacent pixels of the finer level, inside from
-// 3 x 4 outputs (columns, then rows).  (The adjoint takes sides of 16 and more,
-// so levels of fewer than 5 rows or columns come from coarse scales only: those
-// go output by output.)  Scattering 25 atomics per output took 55 + 19 us for
-// the two steps of 16 x 512 x 512 (six scales), this 24 + 13.
+// 3 x 4 outputs (columns, then rows).  Scattering 25 atomics per output took
+// 55 + 19 us for the two steps of 16 x 512 x 512 (six scales), this 24 + 13.
 __global__ void __launch_bounds__(256) k_pyr_down_f_adj(const PyrJobF* __restrict__ jobs) {
   const PyrJobF j = jobs[blockIdx.z];
   const int x = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
   if (x >= j.sw || y >= j.sh) return;
   float* __restrict__ dst = j.dst + (size_t)y * j.dp + x;
-  if (j.sw >= 5 && j.sh >= 5) {
-    float wy[3];
-    const int Y0 = pyr_adj_weights(y, j.sh, wy);
-    if (x >= 4 && x + 8 < j.sw) {   // no border in x
-      float4 d = *reinterpret_cast<const float4*>(dst);
-      const float* src = j.src + (x >> 1) - 1;
-      float v[4] = {0.f, 0.f, 0.f, 0.f};   // columns x/2 - 1 .. x/2 + 2
+  float wy[3];
+  const int Y0 = pyr_adj_weights(y, j.sh, wy);
+  if (x >= 4 && x + 8 < j.sw) {   // no border in x
+    float4 d = *reinterpret_cast<const float4*>(dst);
+    const float* src = j.src + (x >> 1) - 1;
+    float v[4] = {0.f, 0.f, 0.f, 0.f};   // columns x/2 - 1 .. x/2 + 2
 #pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        if (wy[i] == 0.f) continue;
-        const float* row = src + (size_t)(Y0 + i) * j.sp;
-        const float2 m = __ldg(reinterpret_cast<const float2*>(row + 1));   // x/2 is even
-        const float c[4] = {__ldg(row), m.x, m.y, __ldg(row + 3)};
+    for (int i = 0; i < 3; ++i) {
+      if (wy[i] == 0.f) continue;
+      const float* row = src + (size_t)(Y0 + i) * j.sp;
+      const float2 m = __ldg(reinterpret_cast<const float2*>(row + 1));   // x/2 is even
+      const float c[4] = {__ldg(row), m.x, m.y, __ldg(row + 3)};
 #pragma unroll
-        for (int k = 0; k < 4; ++k) v[k] = fmaf(wy[i], c[k], v[k]);
-      }
-      constexpr float s1 = 1.f / 256.f, s4 = 4.f / 256.f, s6 = 6.f / 256.f;
-      d.x += s1 * (v[0] + v[2]) + s6 * v[1];
-      d.y += s4 * (v[1] + v[2]);
-      d.z += s1 * (v[1] + v[3]) + s6 * v[2];
-      d.w += s4 * (v[2] + v[3]);
-      *reinterpret_cast<float4*>(dst) = d;
-      return;
+      for (int k = 0; k < 4; ++k) v[k] = fmaf(wy[i], c[k], v[k]);
     }
-    for (int e = 0; e < 4 && x + e < j.sw; ++e) {
-      float wx[3], acc = 0.f;
-      const int X0 = pyr_adj_weights(x + e, j.sw, wx);
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-          if (wy[i] != 0.f && wx[k] != 0.f)
-            acc = fmaf(wy[i] * wx[k], __ldg(j.src + (size_t)(Y0 + i) * j.sp + X0 + k), acc);
-      dst[e] += acc * (1.0f / 256.0f);
-    }
+    constexpr float s1 = 1.f / 256.f, s4 = 4.f / 256.f, s6 = 6.f / 256.f;
+    d.x += s1 * (v[0] + v[2]) + s6 * v[1];
+    d.y += s4 * (v[1] + v[2]);
+    d.z += s1 * (v[1] + v[3]) + s6 * v[2];
+    d.w += s4 * (v[2] + v[3]);
+    *reinterpret_cast<float4*>(dst) = d;
     return;
   }
-  const float w5[5] = {1.f, 4.f, 6.f, 4.f, 1.f};
   for (int e = 0; e < 4 && x + e < j.sw; ++e) {
-    float acc = 0.f;
-    for (int Y = 0; Y < j.dh; ++Y)
-      for (int i = 0; i < 5; ++i)
-        if (reflect101(2 * Y + i - 2, j.sh) == y)
-          for (int X = 0; X < j.dw; ++X)
-            for (int k = 0; k < 5; ++k)
-              if (reflect101(2 * X + k - 2, j.sw) == x + e) acc += w5[i] * w5[k] * j.src[(size_t)Y * j.sp + X];
+    float wx[3], acc = 0.f;
+    const int X0 = pyr_adj_weights(x + e, j.sw, wx);
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+        if (wy[i] != 0.f && wx[k] != 0.f)
+          acc = fmaf(wy[i] * wx[k], __ldg(j.src + (size_t)(Y0 + i) * j.sp + X0 + k), acc);
     dst[e] += acc * (1.0f / 256.0f);
   }
 }
