@@ -87,11 +87,15 @@ _PROTOS = [
                                            C.c_void_p, C.c_size_t, C.c_int, C.c_void_p, C.c_void_p]),
     ("bimp_detect_host", C.c_int, [C.c_void_p, C.c_void_p, C.c_size_t, C.c_int, C.c_int,
                                    C.POINTER(KeyPointC), C.c_int, C.POINTER(C.c_int), C.c_void_p]),
+    ("bimp_detect_host_staged", C.c_int, [C.c_void_p, C.c_void_p, C.c_size_t, C.c_int, C.c_int, C.c_int,
+                                          C.POINTER(C.POINTER(KeyPointC)), C.POINTER(C.c_int), C.c_void_p]),
     ("bimp_pipeline_create", C.c_int, [C.POINTER(C.c_void_p), C.c_int, C.c_int, C.POINTER(C.c_float), C.c_int,
                                        C.POINTER(Params), C.c_int, C.c_int]),
     ("bimp_pipeline_destroy", C.c_int, [C.c_void_p]),
     ("bimp_pipeline_push", C.c_int, [C.c_void_p, C.c_void_p, C.c_size_t, C.c_int, C.c_int]),
     ("bimp_pipeline_pop", C.c_int, [C.c_void_p, C.POINTER(KeyPointC), C.c_int, C.POINTER(C.c_int)]),
+    ("bimp_pipeline_pop_staged", C.c_int, [C.c_void_p, C.c_int, C.POINTER(C.POINTER(KeyPointC)),
+                                           C.POINTER(C.c_int)]),
     ("bimp_pipeline_in_flight", C.c_int, [C.c_void_p]),
     ("bimp_dense_map", C.c_int, [C.c_void_p, C.c_int, C.c_int, C.c_void_p, C.c_size_t, C.c_void_p]),
     ("bimp_complex_map", C.c_int, [C.c_void_p, C.c_int, C.c_int, C.c_void_p, C.c_size_t, C.c_void_p]),

@@ -231,28 +231,28 @@ _HOST_RECORD = np.dtype([("x", "<f4"), ("y", "<f4"), ("size", "<f4"), ("angle", 
                          ("octave", "<i4"), ("class_id", "<i4")])
 
 
-def _host_records(capacity: int):
-    """A new array for `capacity` records and its pointer: the library writes
-    the records straight into the array that the caller gets (its first part).
-    Pages that no record reaches are never touched; a zeroed ctypes array of
-    the capacity and a copy out of it took more than half of a 1080p
-    detect_host call."""
-    out = np.empty(max(capacity, 1), dtype=_HOST_RECORD)
-    return out, C.cast(out.ctypes.data, C.POINTER(L.KeyPointC))
+def _own_records(staged, n: int) -> np.ndarray:
+    """An array of the n records at `staged` (the library's pinned staging), which
+    the caller owns: exactly as large as what was found.  (A zeroed ctypes array of
+    the capacity and two copies took more than half of a 1080p detect_host call.)"""
+    out = np.empty(n, dtype=_HOST_RECORD)
+    if n > 0:
+        C.memmove(out.ctypes.data, staged, out.nbytes)
+    return out
 
 
 def detect_host(cs: CudaStuff, image: np.ndarray, capacity: int = KP_MAX_POINTS):
-    """Host image in, host records out through bimp_detect_host.
+    """Host image in, host records out through bimp_detect_host_staged.
 
     Returns (structured array of cv::KeyPoint fields, total count, status)."""
     img = np.ascontiguousarray(image, dtype=np.uint8)
-    out, ptr = _host_records(capacity)
+    staged = C.POINTER(L.KeyPointC)()
     n = C.c_int(0)
-    rc = L.lib().bimp_detect_host(cs.handle, C.c_void_p(img.ctypes.data), img.strides[0], img.shape[1],
-                                  img.shape[0], ptr, capacity, C.byref(n), _stream_ptr())
+    rc = L.lib().bimp_detect_host_staged(cs.handle, C.c_void_p(img.ctypes.data), img.strides[0], img.shape[1],
+                                         img.shape[0], capacity, C.byref(staged), C.byref(n), _stream_ptr())
     if rc not in (L.BIMP_OK, L.BIMP_ERR_CAPACITY):
         L.check(rc, "detect_host")
-    return out[:min(n.value, capacity)], n.value, rc
+    return _own_records(staged, min(n.value, capacity)), n.value, rc
 
 
 def min_size_dims(width: int, height: int) -> tuple:
@@ -432,13 +432,13 @@ class Pipeline:
     def pop(self, capacity: int | None = None):
         """(records, total, status) of the oldest frame in flight."""
         cap = self.capacity if capacity is None else int(capacity)
-        out, ptr = _host_records(min(cap, self.capacity))
+        staged = C.POINTER(L.KeyPointC)()
         n = C.c_int(0)
-        rc = L.lib().bimp_pipeline_pop(self._h, ptr, cap, C.byref(n))
+        rc = L.lib().bimp_pipeline_pop_staged(self._h, cap, C.byref(staged), C.byref(n))
         if rc not in (L.BIMP_OK, L.BIMP_ERR_CAPACITY):
             L.check(rc, "pipeline_pop")
         self._frames.pop(0)
-        return out[:min(n.value, cap, self.capacity)], n.value, rc
+        return _own_records(staged, min(n.value, cap, self.capacity)), n.value, rc
 
     def close(self):
         if getattr(self, "_h", None) is not None:

@@ -893,9 +893,9 @@ static int host_enqueue(bimp_context* c, const uint8_t* image, size_t pitch, int
 
 // Host path, second half, once stream s has finished the first: the records
 // beyond the speculative copy (rare: a count well above the previous call's)
-// come back with one more copy and synchronisation, then everything is
-// copied from the staging into the caller's array.
-static int host_finish(bimp_context* c, int spec, bimp_keypoint* out, int capacity, int* n_found, cudaStream_t s) {
+// come back with one more copy and synchronisation.  The first min(*n_found,
+// capacity) records are then in the pinned staging.
+static int host_finish(bimp_context* c, int spec, int capacity, int* n_found, cudaStream_t s) {
   const int total = c->h_count[1];
   *n_found = total;
   if (c->h_count[0]) return fail(BIMP_ERR_CUDA, "a bounded device wait expired");
@@ -906,23 +906,39 @@ static int host_finish(bimp_context* c, int spec, bimp_keypoint* out, int capaci
     BIMP_CUDA(cudaStreamSynchronize(s));
   }
   static_assert(sizeof(bimp_keypoint) == 7 * sizeof(float), "record layout");
-  if (n > 0) std::memcpy(out, c->h_stage, sizeof(bimp_keypoint) * (size_t)n);
   c->specRecords = std::max(256, std::min(std::max(capacity, 1), n + n / 8 + 256));
   if (total > capacity)
     return fail(BIMP_ERR_CAPACITY, "keypoints exceed capacity (" + std::to_string(total) + ")");
   return BIMP_OK;
 }
 
-int bimp_detect_host(bimp_context* c, const uint8_t* image, size_t pitch, int width, int height,
-                     bimp_keypoint* out, int capacity, int* n_found, void* stream) {
-  if (!c || !n_found || capacity < 0 || (capacity > 0 && !out))
-    return fail(BIMP_ERR_INVALID, "null argument");
+// From the staging into the caller's array, where the call has records.
+static void host_copy(const bimp_keypoint* staged, bimp_keypoint* out, int rc, int n_found, int capacity) {
+  const int n = std::min(n_found, capacity);
+  if ((rc == BIMP_OK || rc == BIMP_ERR_CAPACITY) && n > 0) std::memcpy(out, staged, sizeof(bimp_keypoint) * (size_t)n);
+}
+
+int bimp_detect_host_staged(bimp_context* c, const uint8_t* image, size_t pitch, int width, int height, int capacity,
+                            const bimp_keypoint** records, int* n_found, void* stream) {
+  if (!c || !records || !n_found || capacity < 0) return fail(BIMP_ERR_INVALID, "null argument");
+  *records = nullptr;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   int spec = 0;
   const int rc = host_enqueue(c, image, pitch, width, height, capacity, s, &spec);
   if (rc != BIMP_OK) return rc;
   BIMP_CUDA(cudaStreamSynchronize(s));
-  return host_finish(c, spec, out, capacity, n_found, s);
+  *records = c->h_stage;
+  return host_finish(c, spec, capacity, n_found, s);
+}
+
+int bimp_detect_host(bimp_context* c, const uint8_t* image, size_t pitch, int width, int height,
+                     bimp_keypoint* out, int capacity, int* n_found, void* stream) {
+  if (!c || !n_found || capacity < 0 || (capacity > 0 && !out))
+    return fail(BIMP_ERR_INVALID, "null argument");
+  const bimp_keypoint* staged = nullptr;
+  const int rc = bimp_detect_host_staged(c, image, pitch, width, height, capacity, &staged, n_found, stream);
+  if (staged) host_copy(staged, out, rc, *n_found, capacity);
+  return rc;
 }
 
 int bimp_dense_map(bimp_context* c, int scale, int which, float* d_out, size_t ld, void* stream) {
@@ -1332,8 +1348,9 @@ int bimp_pipeline_push(bimp_pipeline* p, const uint8_t* image, size_t pitch, int
   return BIMP_OK;
 }
 
-int bimp_pipeline_pop(bimp_pipeline* p, bimp_keypoint* out, int capacity, int* n_found) {
-  if (!p || !n_found || capacity < 0 || (capacity > 0 && !out)) return fail(BIMP_ERR_INVALID, "null argument");
+int bimp_pipeline_pop_staged(bimp_pipeline* p, int capacity, const bimp_keypoint** records, int* n_found) {
+  if (!p || !records || !n_found || capacity < 0) return fail(BIMP_ERR_INVALID, "null argument");
+  *records = nullptr;
   if (p->inFlight == 0) return fail(BIMP_ERR_INVALID, "no frame in flight");
   const int k = p->head;
   p->head = (p->head + 1) % p->depth;
@@ -1341,13 +1358,22 @@ int bimp_pipeline_pop(bimp_pipeline* p, bimp_keypoint* out, int capacity, int* n
   BIMP_CUDA(cudaSetDevice(p->device));
   BIMP_CUDA(cudaEventSynchronize(p->done[k]));
   int total = 0;
-  const int rc = host_finish(p->ctx[k], p->spec[k], out, std::min(capacity, p->capacity), &total, p->streams[k]);
+  const int rc = host_finish(p->ctx[k], p->spec[k], std::min(capacity, p->capacity), &total, p->streams[k]);
+  *records = p->ctx[k]->h_stage;
   *n_found = total;
   if (rc == BIMP_ERR_CAPACITY && total <= capacity) {
     // more than the pipeline's own capacity was found: the records beyond it
     // were never written
     return fail(BIMP_ERR_CAPACITY, "keypoints exceed the pipeline capacity (" + std::to_string(total) + ")");
   }
+  return rc;
+}
+
+int bimp_pipeline_pop(bimp_pipeline* p, bimp_keypoint* out, int capacity, int* n_found) {
+  if (!p || !n_found || capacity < 0 || (capacity > 0 && !out)) return fail(BIMP_ERR_INVALID, "null argument");
+  const bimp_keypoint* staged = nullptr;
+  const int rc = bimp_pipeline_pop_staged(p, capacity, &staged, n_found);
+  if (staged) host_copy(staged, out, rc, *n_found, std::min(capacity, p->capacity));
   return rc;
 }
 

@@ -158,6 +158,15 @@ int bimp_detect_host(bimp_context* ctx, const uint8_t* image, size_t pitch,
                      int width, int height, bimp_keypoint* out, int capacity,
                      int* n_found, void* stream);
 
+/* The same without a copy into the caller's memory: *records is the context's
+ * pinned staging, whose first min(*n_found, capacity) records are the call's
+ * (BIMP_OK or BIMP_ERR_CAPACITY).  They stay until the next host call on the
+ * context.  A caller that allocates its array for the count found copies them
+ * from there once. */
+int bimp_detect_host_staged(bimp_context* ctx, const uint8_t* image, size_t pitch,
+                            int width, int height, int capacity,
+                            const bimp_keypoint** records, int* n_found, void* stream);
+
 /* ---- pipelined host frames (no counterpart in the reference) -------------
  * The reference handles one frame per call and synchronises the device at
  * entry and exit (bimp/src/bimp.cpp:62, bimp/src/cuda_bimp.cu:115), so a
@@ -183,6 +192,10 @@ int bimp_pipeline_push(bimp_pipeline* pipeline, const uint8_t* image, size_t pit
 /* Records of the oldest frame in flight, in (scale, y, x) order;
  * BIMP_ERR_INVALID when no frame is in flight. */
 int bimp_pipeline_pop(bimp_pipeline* pipeline, bimp_keypoint* out, int capacity, int* n_found);
+/* The same, the records left in the frame's pinned staging (see
+ * bimp_detect_host_staged): min(*n_found, capacity, the pipeline's capacity) of
+ * them, until the next push. */
+int bimp_pipeline_pop_staged(bimp_pipeline* pipeline, int capacity, const bimp_keypoint** records, int* n_found);
 int bimp_pipeline_in_flight(const bimp_pipeline* pipeline);
 
 /* Per-scale dense maps of the last detection (Context::getResponses,
