@@ -117,6 +117,9 @@ _PROTOS = [
     ("bimp_upload_keypoints", C.c_int, [C.POINTER(KeyPointC), C.c_int, C.c_void_p, C.c_size_t, C.c_void_p]),
     ("bimp_adjoint_create", C.c_int, [C.POINTER(C.c_void_p), C.c_int, C.c_int, C.c_int, C.POINTER(C.c_float),
                                       C.c_int, C.POINTER(Params)]),
+    ("bimp_adjoint_create_keep", C.c_int, [C.POINTER(C.c_void_p), C.c_int, C.c_int, C.c_int, C.POINTER(C.c_float),
+                                           C.c_int, C.POINTER(Params), C.c_size_t]),
+    ("bimp_adjoint_kept_bytes", C.c_size_t, [C.c_void_p]),
     ("bimp_adjoint_destroy", C.c_int, [C.c_void_p]),
     ("bimp_adjoint_num_scales", C.c_int, [C.c_void_p]),
     ("bimp_adjoint_mask_layout", C.c_int, [C.c_void_p, C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_int),

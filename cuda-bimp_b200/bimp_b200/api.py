@@ -572,14 +572,21 @@ class Adjoint:
     forward(images, masks) -> loss; backward() -> (dL/dimages, dL/d(alpha,
     rho, w_tan, w_rad)).  images: float32 CUDA tensor (n, H, W); masks: float32
     CUDA tensor of n * mask_stride elements laid out by mask_views().
+
+    keep_bytes: the most device memory that the forward may keep its responses
+    in for the backward, which otherwise recomputes them in about 1.4 times the
+    time (0: none; kept_bytes() says what was taken).  The memory is the library's,
+    not torch's allocator's, held until close().  Default: up to 8 GiB and an
+    eighth of what is free when the object is made.
     """
 
-    def __init__(self, width: int, height: int, n_images: int, lambdas, params=None):
+    def __init__(self, width: int, height: int, n_images: int, lambdas, params=None, keep_bytes: int | None = None):
         lam = (C.c_float * len(lambdas))(*[float(x) for x in lambdas])
         p = _params(params)
         h = C.c_void_p()
-        L.check(L.lib().bimp_adjoint_create(C.byref(h), int(width), int(height), int(n_images), lam, len(lambdas),
-                                            C.byref(p) if p is not None else None), "Adjoint")
+        keep = C.c_size_t(-1).value if keep_bytes is None else max(0, int(keep_bytes))
+        L.check(L.lib().bimp_adjoint_create_keep(C.byref(h), int(width), int(height), int(n_images), lam, len(lambdas),
+                                                 C.byref(p) if p is not None else None, keep), "Adjoint")
         self._h = h
         self.params = p if p is not None else default_params()
         self.width, self.height, self.n = int(width), int(height), int(n_images)
@@ -637,6 +644,10 @@ class Adjoint:
         L.check(L.lib().bimp_adjoint_complex_map(self._h, image, scale, orientation, C.c_void_p(out.data_ptr()),
                                                  out.stride(0), _stream_ptr()), "adjoint_complex_map")
         return out
+
+    def kept_bytes(self) -> int:
+        """Device memory that the forward keeps responses in (0: none)."""
+        return int(L.lib().bimp_adjoint_kept_bytes(self._h))
 
     def device_bytes(self) -> int:
         return int(L.lib().bimp_adjoint_device_bytes(self._h))

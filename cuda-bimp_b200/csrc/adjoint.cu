@@ -110,11 +110,13 @@ struct bimp_adjoint {
   unsigned int* d_fault = nullptr;        // bits set by the kernels when a bounded wait expired, until status() reads them
 
   // Memory for the forward's e + i o and tile spectra, which let the backward
-  // start from them instead of transforming every tile again.  It is taken
-  // where the program has plenty: up to kKeepBudget and an eighth of the
-  // device's free memory (BIMP_ADJOINT_KEEP=0: none, for tests); otherwise, or
-  // if it cannot be had, the backward recomputes both.
-  void reserve_kept(const std::vector<ScaleDev>& sds, std::vector<size_t>& offZ, std::vector<size_t>& offX) {
+  // start from them instead of transforming every tile again: up to the
+  // caller's limit.  Without one it is taken where the program has
+  // plenty: up to kKeepBudget and an eighth of the device's free memory
+  // (BIMP_ADJOINT_KEEP=0: none, for tests).  Beyond that, or if it cannot be had,
+  // the backward recomputes both.
+  void reserve_kept(const std::vector<ScaleDev>& sds, size_t limit, std::vector<size_t>& offZ,
+                    std::vector<size_t>& offX) {
     size_t at = 0;
     for (const ScaleDev& d : sds) {
       offZ.push_back(at);
@@ -122,11 +124,14 @@ struct bimp_adjoint {
       offX.push_back(at);
       at += up(sizeof(float2) * kSpecHalf * (size_t)d.tilesX * d.tilesY, 256);
     }
-    constexpr size_t kKeepBudget = size_t(8) << 30;
-    size_t freeB = 0, totalB = 0;
-    const char* k = std::getenv("BIMP_ADJOINT_KEEP");
-    if ((k && std::atoi(k) == 0) || cudaMemGetInfo(&freeB, &totalB) != cudaSuccess) return;
-    if (at > kKeepBudget || at > freeB / 8) return;
+    if (limit == BIMP_ADJOINT_KEEP_AUTO) {
+      constexpr size_t kKeepBudget = size_t(8) << 30;
+      size_t freeB = 0, totalB = 0;
+      const char* k = std::getenv("BIMP_ADJOINT_KEEP");
+      if ((k && std::atoi(k) == 0) || cudaMemGetInfo(&freeB, &totalB) != cudaSuccess) return;
+      limit = std::min(kKeepBudget, freeB / 8);
+    }
+    if (at > limit) return;
     if (cudaMalloc(&keep, at) != cudaSuccess) {
       cudaGetLastError();
       keep = nullptr;
@@ -135,7 +140,7 @@ struct bimp_adjoint {
     keepBytes = at;
   }
 
-  int build(int dev, int w, int h, int ni, const float* lambdas, int nl, const bimp_params& p) {
+  int build(int dev, int w, int h, int ni, const float* lambdas, int nl, const bimp_params& p, size_t keepLimit) {
     device = dev;
     W = w;
     H = h;
@@ -280,7 +285,7 @@ struct bimp_adjoint {
     pipelined = kern && std::strcmp(kern, "pipelined") == 0;
     for (const ScaleDev& d : sds) pipelined = pipelined && d.V <= pipelined_tile_max_valid();
     std::vector<size_t> offZ, offX;   // per entry, in `keep`
-    if (!pipelined) reserve_kept(sds, offZ, offX);
+    if (!pipelined) reserve_kept(sds, keepLimit, offZ, offX);
     std::vector<TileWork> plans;
     // CTAs of the plans: one per SM (BIMP_ADJOINT_GRID overrides it, for tests:
     // on a few CTAs small images too make items of several orientations and
@@ -464,8 +469,8 @@ struct bimp_adjoint {
 
 extern "C" {
 
-int bimp_adjoint_create(bimp_adjoint** out, int width, int height, int n_images, const float* lambdas,
-                        int n_lambdas, const bimp_params* params) {
+int bimp_adjoint_create_keep(bimp_adjoint** out, int width, int height, int n_images, const float* lambdas,
+                             int n_lambdas, const bimp_params* params, size_t keep_bytes) {
   if (!out) return afail(BIMP_ERR_INVALID, "out is null");
   *out = nullptr;
   if (width < 16 || height < 16 || n_images <= 0 || !lambdas || n_lambdas <= 0)
@@ -479,7 +484,7 @@ int bimp_adjoint_create(bimp_adjoint** out, int width, int height, int n_images,
   int rc = configure_device(dev);
   if (rc != BIMP_OK) return rc;
   bimp_adjoint* a = new bimp_adjoint();
-  rc = a->build(dev, width, height, n_images, lambdas, n_lambdas, p);
+  rc = a->build(dev, width, height, n_images, lambdas, n_lambdas, p, keep_bytes);
   if (rc != BIMP_OK) {
     if (a->mem) cudaFree(a->mem);
     if (a->keep) cudaFree(a->keep);
@@ -488,6 +493,11 @@ int bimp_adjoint_create(bimp_adjoint** out, int width, int height, int n_images,
   }
   *out = a;
   return BIMP_OK;
+}
+
+int bimp_adjoint_create(bimp_adjoint** out, int width, int height, int n_images, const float* lambdas,
+                        int n_lambdas, const bimp_params* params) {
+  return bimp_adjoint_create_keep(out, width, height, n_images, lambdas, n_lambdas, params, BIMP_ADJOINT_KEEP_AUTO);
 }
 
 int bimp_adjoint_destroy(bimp_adjoint* a) {
@@ -500,6 +510,8 @@ int bimp_adjoint_destroy(bimp_adjoint* a) {
 }
 
 int bimp_adjoint_num_scales(const bimp_adjoint* a) { return a ? a->nScales : 0; }
+
+size_t bimp_adjoint_kept_bytes(const bimp_adjoint* a) { return a ? a->keepBytes : 0; }
 
 size_t bimp_adjoint_device_bytes(const bimp_adjoint* a) { return a ? a->bytes + a->keepBytes : 0; }
 

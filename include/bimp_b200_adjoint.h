@@ -22,8 +22,11 @@
  * magnitude has no derivative; the value assumes images on the [0, 1] scale).
  * The forward keeps the complex responses and each tile's image spectrum
  * for the backward where the adjoint got the memory for them when it was
- * created (up to 8 GiB and an eighth of the device's free memory); otherwise
- * the backward recomputes them, with the same results.
+ * created; otherwise the backward recomputes them, with the same results, in
+ * about 1.4 times the time.  It is all images' or none's, allocated
+ * by the library and held until the adjoint is destroyed: up to 8 GiB and an
+ * eighth of the device's memory that is free at that moment, or up to what the
+ * caller allows (bimp_adjoint_create_keep).
  */
 #ifndef BIMP_B200_ADJOINT_H
 #define BIMP_B200_ADJOINT_H
@@ -39,6 +42,11 @@ typedef struct bimp_adjoint bimp_adjoint;
 /* n_images float images of width x height, one wavelength bank. */
 int bimp_adjoint_create(bimp_adjoint** out, int width, int height, int n_images, const float* lambdas,
                         int n_lambdas, const bimp_params* params);
+/* The same with the caller's limit on the memory that the forward may keep
+ * responses in: at most keep_bytes (0: none). */
+#define BIMP_ADJOINT_KEEP_AUTO ((size_t)-1)
+int bimp_adjoint_create_keep(bimp_adjoint** out, int width, int height, int n_images, const float* lambdas,
+                             int n_lambdas, const bimp_params* params, size_t keep_bytes);
 int bimp_adjoint_destroy(bimp_adjoint* a);
 int bimp_adjoint_num_scales(const bimp_adjoint* a);
 
@@ -79,7 +87,11 @@ int bimp_adjoint_dense_map(bimp_adjoint* a, int image, int scale, float* d_out, 
 int bimp_adjoint_complex_map(bimp_adjoint* a, int image, int scale, int orientation, float* d_out, size_t ld,
                              void* stream);
 
-/* Device bytes held by the adjoint's buffers. */
+/* Bytes of the memory that the forward keeps responses in (0: the backward
+ * recomputes them). */
+size_t bimp_adjoint_kept_bytes(const bimp_adjoint* a);
+
+/* Device bytes held by the adjoint's buffers, the kept responses among them. */
 size_t bimp_adjoint_device_bytes(const bimp_adjoint* a);
 
 #ifdef __cplusplus
