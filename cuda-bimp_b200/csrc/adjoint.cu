@@ -84,11 +84,8 @@ struct bimp_adjoint {
   };
   std::vector<Plan> fwdPlan, bwdPlan;
   TileWork* d_tiles = nullptr;
-  int nTiles = 0;
   int2* d_sten = nullptr;                 // forward stencil blocks (data)
-  int nSten = 0;
   int2* d_stenB = nullptr;                // backward gather blocks (window rows 0..dataH+1)
-  int nStenB = 0;
   std::vector<float*> lvl, glvl;          // [level][image]
   std::vector<int> lw, lh, lp;            // per level (same for all images)
   float* d_lvl0 = nullptr;                // level 0 of every image, n * H rows of lp[0]
@@ -277,9 +274,6 @@ struct bimp_adjoint {
     tileStart.push_back(static_cast<int>(tiles.size()));
     stenStart.push_back(static_cast<int>(sten.size()));
     stenBStart.push_back(static_cast<int>(stenB.size()));
-    nTiles = static_cast<int>(tiles.size());
-    nSten = static_cast<int>(sten.size());
-    nStenB = static_cast<int>(stenB.size());
     // the kernel that pipelines the forward (BIMP_TILE_KERNEL=pipelined) keeps nothing
     const char* kern = std::getenv("BIMP_TILE_KERNEL");
     pipelined = kern && std::strcmp(kern, "pipelined") == 0;

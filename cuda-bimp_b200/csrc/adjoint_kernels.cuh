@@ -270,7 +270,7 @@ constexpr float kMagFloor = 3.0e-5f;
 __device__ __forceinline__ int perm128d(int k) { return 8 * (k & 15) + (k >> 4); }
 
 // Persistent CTAs walk the work items, each a tile and a run of its
-// orientations (one CTA per SM: 223 KB of shared memory and all 512 TMEM
+// orientations (one CTA per SM: 222 KiB of shared memory and all 512 TMEM
 // columns).  The window gradient is linear in the per-orientation spectra,
 // Re IFFT(sum_o A_o G_o), so the products are summed in the frequency domain
 // (Hermitian half, Bh) and ONE inverse transform per item replaces one per

@@ -863,8 +863,7 @@ static_assert(2 * kWsRows >= 193, "forward-transform scratch does not fit the ro
 constexpr int kWsGroup = kTileThreads / 2;   // threads per group
 enum : int { kBarY = 1, kBarX = 2, kBarFull0 = 3, kBarEmpty0 = 5 };   // named barrier ids (0 is __syncthreads)
 
-__device__ __forceinline__ void nbar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
-__device__ __forceinline__ void nbar_arrive(int id, int n) {
+__device__ __forceinline__ void named_barrier_arrive(int id, int n) {
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory");
 }
 
@@ -945,9 +944,9 @@ k_gabor_tiles_ws(const ScaleDev* __restrict__ sds, const TileWork* __restrict__ 
         }
         tmem_wait_st();
         tmem_fence_before();
-        nbar_sync(kBarY, kWsGroup);   // the y-area holds orientation o's first y-pass
+        named_barrier(kBarY, kWsGroup);   // the y-area holds orientation o's first y-pass
         tmem_fence_after();
-        if (o - oB >= 2) nbar_sync(kBarEmpty0 + b, kTileThreads);   // group X is done with orientation o - 2
+        if (o - oB >= 2) named_barrier(kBarEmpty0 + b, kTileThreads);   // group X is done with orientation o - 2
         // I2: y-dim pass A' -> natural y; the valid rows into buffer b
 #pragma unroll
         for (int it = 0; it < 4; ++it) {
@@ -963,8 +962,8 @@ k_gabor_tiles_ws(const ScaleDev* __restrict__ sds, const TileWork* __restrict__ 
           }
         }
         tmem_fence_before();
-        nbar_arrive(kBarFull0 + b, kTileThreads);   // buffer b holds orientation o
-        nbar_sync(kBarY, kWsGroup);                 // every thread is done reading the y-area
+        named_barrier_arrive(kBarFull0 + b, kTileThreads);   // buffer b holds orientation o
+        named_barrier(kBarY, kWsGroup);                 // every thread is done reading the y-area
         tmem_fence_after();
       }
     } else {
@@ -985,7 +984,7 @@ k_gabor_tiles_ws(const ScaleDev* __restrict__ sds, const TileWork* __restrict__ 
         const int b = (o - oB) & 1;
         float2* Wo = Wb + b * kWsBuf;
         float* __restrict__ Cout = C0p + (size_t)o * cStride;
-        nbar_sync(kBarFull0 + b, kTileThreads);
+        named_barrier(kBarFull0 + b, kTileThreads);
         // I3: x-dim pass B' on the V rows of the buffer (a thread's k2 is
         // fixed: its twiddles are loaded once)
         {
@@ -1003,7 +1002,7 @@ k_gabor_tiles_ws(const ScaleDev* __restrict__ sds, const TileWork* __restrict__ 
             for (int n1 = 0; n1 < 8; ++n1) Wo[RotLayout::at(y, 8 * k2 + n1)] = n1 ? c_mulc(v[n1], twr[n1]) : v[0];
           }
         }
-        nbar_sync(kBarX, kWsGroup);
+        named_barrier(kBarX, kWsGroup);
         // I4: x-dim pass A' -> natural x; complex magnitude of valid outputs
         for (int j = tg; j < Vr * 8; j += kWsGroup) {
           const int y = j >> 3, n1 = j & 7;
@@ -1037,7 +1036,7 @@ k_gabor_tiles_ws(const ScaleDev* __restrict__ sds, const TileWork* __restrict__ 
         }
         // buffer b may be refilled by orientation o + 2; the item's last two
         // orientations are ordered against the next tile by its barrier
-        if (o - oB < nO - 2) nbar_arrive(kBarEmpty0 + b, kTileThreads);
+        if (o - oB < nO - 2) named_barrier_arrive(kBarEmpty0 + b, kTileThreads);
       }
     }
   }
