@@ -357,7 +357,11 @@ __device__ __forceinline__ void raw_chunks_load(const ScaleDev* sd, int R0, int 
 }
 // The window's columns outside [iA, iB) (which no chunk writes), value by value
 // through the padded-torus map: warp w stages rows w, w + 16, ..., lane l the columns l,
-// l + 32, l + 64, l + 96 among them.
+// l + 32, l + 64, l + 96 among them.  Bound by the latency of its loads: a group
+// of columns at a time (most windows have one or two with columns outside), the
+// loads of its eight rows in flight together.  All four groups of four rows at
+// once took registers that the pipelined kernel spilled: 4 images of 512 x 512
+// 139 us a detection with it and 134 so, 112 and 111 with k_gabor_tiles.
 template <bool FLT>
 __device__ __forceinline__ void raw_window_copy(const ScaleDev* sd, int R0, int C0, typename RawWindow<FLT>::T* raw,
                                                 int iA, int iB, int t) {
@@ -369,31 +373,19 @@ __device__ __forceinline__ void raw_window_copy(const ScaleDev* sd, int R0, int 
   if constexpr (FLT) { lvl = sd->lvlF; pitch = sd->lvlPitchF; }
   else { lvl = sd->lvl; pitch = sd->lvlPitch; }
   const int myRow = window_src(R0 - kX, w0 + 16 * (lane & 7), sd->fftH, sd->dataH, kX);
-  int c[4];
-  bool mine[4], any[4];
-#pragma unroll
+#pragma unroll 1
   for (int k = 0; k < 4; ++k) {
     const int i = lane + 32 * k;
-    mine[k] = i < iA || i >= iB;
-    any[k] = __any_sync(0xffffffffu, mine[k]);
-    c[k] = any[k] ? window_src(C0 - kX, i, sd->fftW, sd->dataW, kX) : 0;
-  }
-  constexpr int kBatch = 4;   // rows whose loads are in flight together (eight: spills in the pipelined kernel)
-#pragma unroll 1
-  for (int i0 = 0; i0 < 8; i0 += kBatch) {
-    T v[kBatch][4];
+    const bool mine = i < iA || i >= iB;
+    if (!__any_sync(0xffffffffu, mine)) continue;
+    const int c = window_src(C0 - kX, i, sd->fftW, sd->dataW, kX);
+    T v[8];
 #pragma unroll
-    for (int i = 0; i < kBatch; ++i) {
-      const T* row = lvl + (size_t)__shfl_sync(0xffffffffu, myRow, i0 + i) * pitch;
+    for (int r = 0; r < 8; ++r) v[r] = lvl[(size_t)__shfl_sync(0xffffffffu, myRow, r) * pitch + c];
+    if (mine) {
 #pragma unroll
-      for (int k = 0; k < 4; ++k)
-        if (any[k]) v[i][k] = row[c[k]];
+      for (int r = 0; r < 8; ++r) raw[(w0 + 16 * r) * P + i] = v[r];
     }
-#pragma unroll
-    for (int i = 0; i < kBatch; ++i)
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-        if (any[k] && mine[k]) raw[(w0 + 16 * (i0 + i)) * P + lane + 32 * k] = v[i][k];
   }
 }
 
@@ -849,9 +841,9 @@ k_gabor_tiles(const ScaleDev* __restrict__ sds, const TileWork* __restrict__ wor
 // barrier stands inside the orientation loop.  G_o is read from L2 (the
 // second buffer takes the space it would be staged in), a thread's eight values
 // as two 16-byte loads.  Needs V <= kWsRows.  64 mixed images, one CTA a tile:
-// 7.62 ms a detection (8.69 with the values loaded one by one in the order of
+// 7.47 ms a detection (8.69 with the values loaded one by one in the order of
 // the stored spectrum and the window staged value by value; k_gabor_tiles
-// 6.90).
+// 6.87).
 constexpr int kWsRows = 104;                                  // largest V this kernel takes
 constexpr int kWsBuf = kWsRows * kTile;                       // complex per row buffer
 constexpr int kWsSmemW = 2 * kWsBuf * 8;                      // both row buffers (also the forward scratch)
