@@ -297,7 +297,7 @@ struct bimp_adjoint {
         to.push_back(p);
         return p.grid;
       };
-      add(fwdPlan, kForwardCost);
+      add(fwdPlan, pipelined ? kPipelinedCost : kForwardCost);
       bwdGrid = std::max(bwdGrid, add(bwdPlan, keep ? kBackwardKeptCost : kBackwardCost));
     }
     const size_t offSd = take(sizeof(ScaleDev) * sds.size());

@@ -187,18 +187,19 @@ struct Engine {
   }
   // The tile kernel's work list of a plan: one item per tile (grid <= 0, one
   // CTA each) or the balanced split plan for `grid` persistent CTAs.
-  static std::vector<TileWork> work_list(std::vector<ScaleDev>& sds, int policy, int order, int grid, int* nTilesOut,
-                                         int* gridOut) {
+  static std::vector<TileWork> work_list(std::vector<ScaleDev>& sds, int policy, int order, int grid, bool pipelined,
+                                         int* nTilesOut, int* gridOut) {
     std::vector<TileWork> tiles = tile_plan(sds, policy, order);
     *nTilesOut = static_cast<int>(tiles.size());
     *gridOut = static_cast<int>(tiles.size());
-    if (grid > 0 && !tiles.empty()) return split_plan(tiles, sds, kForwardCost, grid, gridOut);
+    if (grid > 0 && !tiles.empty())
+      return split_plan(tiles, sds, pipelined && pipelined_fits(sds) ? kPipelinedCost : kForwardCost, grid, gridOut);
     return tiles;
   }
   int retile(int policy, int order, int grid, int kernel = 0) {
     std::vector<ScaleDev> sds = h_sd;
     int nt = 0, g = 0;
-    const std::vector<TileWork> work = work_list(sds, policy, order, grid, &nt, &g);
+    const std::vector<TileWork> work = work_list(sds, policy, order, grid, kernel == 1, &nt, &g);
     if ((int)work.size() > tileCap) return fail(BIMP_ERR_INVALID, "tile plan larger than its buffer");
     BIMP_CUDA(cudaSetDevice(device));
     BIMP_CUDA(cudaMemcpy(d_sd, sds.data(), sizeof(ScaleDev) * sds.size(), cudaMemcpyHostToDevice));
@@ -211,22 +212,22 @@ struct Engine {
     tileGridReq = grid > 0 ? grid : 0;
     tilePolicy = policy;
     tileOrder = order;
-    tilePipelined = kernel == 1 && pipelined_fits();
+    tilePipelined = kernel == 1 && pipelined_fits(h_sd);
     return BIMP_OK;
   }
   // The warp-specialised tile kernel takes every scale with V up to its row
   // buffers' height.
-  bool pipelined_fits() const {
-    for (const ScaleDev& d : h_sd)
+  static bool pipelined_fits(const std::vector<ScaleDev>& sds) {
+    for (const ScaleDev& d : sds)
       if (d.V > pipelined_tile_max_valid()) return false;
     return true;
   }
   // Default kernel: the phased one (measured faster on the plain 1080p
   // detection); BIMP_TILE_KERNEL=pipelined selects the warp-specialised one,
   // and a batch's tile plan (or its autotuner) may choose either.
-  bool pipelined_by_default() const {
+  static bool pipelined_by_default(const std::vector<ScaleDev>& sds) {
     const char* k = std::getenv("BIMP_TILE_KERNEL");
-    return k && std::strcmp(k, "pipelined") == 0 && pipelined_fits();
+    return k && std::strcmp(k, "pipelined") == 0 && pipelined_fits(sds);
   }
 
   // inW/inH (null: the geometry sizes) are the sizes of the images a
@@ -401,7 +402,9 @@ struct Engine {
     if (const char* g = std::getenv("BIMP_TILE_GRID")) defGrid = std::atoi(g);
     std::vector<TileWork> work = tiles;
     tileGrid = nTiles;
-    if (defGrid > 0 && !tiles.empty()) work = split_plan(tiles, sds, kForwardCost, defGrid, &tileGrid);
+    tilePipelined = pipelined_by_default(sds);
+    if (defGrid > 0 && !tiles.empty())
+      work = split_plan(tiles, sds, tilePipelined ? kPipelinedCost : kForwardCost, defGrid, &tileGrid);
     nWork = static_cast<int>(work.size());
     tileGridReq = std::max(0, defGrid);
     nSten = static_cast<int>(sten.size());
@@ -413,8 +416,8 @@ struct Engine {
       // its CTAs times the most items of one, so that a list of one item a CTA
       // becomes one of two with a small change of the cost model's weights.
       // (Over random batches and grids up to 4000, what the weights of an
-      // earlier kernel accepted with a buffer of half this size, these accept
-      // too; a plan beyond the buffer is refused by retile.)
+      // earlier kernel accepted with a buffer of half this size, those of both
+      // kernels accept too; a plan beyond the buffer is refused by retile.)
       tileCap = nWork;
       int maxTiles = 0;
       const int grids[4] = {0, sms, 2 * sms, defGrid};
@@ -423,7 +426,7 @@ struct Engine {
           for (int g : grids) {
             std::vector<ScaleDev> tmp = sds;
             int nt = 0, ng = 0;
-            tileCap = std::max(tileCap, static_cast<int>(work_list(tmp, policy, order, g, &nt, &ng).size()));
+            tileCap = std::max(tileCap, static_cast<int>(work_list(tmp, policy, order, g, false, &nt, &ng).size()));
             maxTiles = std::max(maxTiles, nt);
           }
       tileCap = 2 * std::max(tileCap, 2 * maxTiles + 6 * sms);
@@ -487,7 +490,6 @@ struct Engine {
       for (size_t e2 = 0; e2 < sds.size(); ++e2) sds[e2].cMap = base + offMaps + e2 * kTensorMapBytes;
     }
     h_sd = sds;
-    tilePipelined = pipelined_by_default();
     d_sd = reinterpret_cast<ScaleDev*>(base + offSd);
     d_tiles = reinterpret_cast<TileWork*>(base + offTiles);
     d_sten = reinterpret_cast<int2*>(base + offSten);
@@ -1146,7 +1148,7 @@ int bimp_batch_autotune(bimp_batch* b, void* stream, int reps, bimp_tile_plan* c
     sms = 148;
   const int grids[3] = {0, sms, 2 * sms};
   // the pipelined kernel takes every scale only when its valid blocks fit
-  const int kernels = b->eng.pipelined_fits() ? 2 : 1;
+  const int kernels = b->eng.pipelined_fits(b->eng.h_sd) ? 2 : 1;
   cudaEvent_t e0, e1;
   BIMP_CUDA(cudaEventCreate(&e0));
   BIMP_CUDA(cudaEventCreate(&e1));

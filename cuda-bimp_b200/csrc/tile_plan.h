@@ -21,6 +21,11 @@ struct TileCost {
 // 0.77 k of 10.4 k cycles.  The weights before the x-passes went warp by warp
 // left a 3840 x 2160 detection's tile kernel at 946 us, these 859.
 constexpr TileCost kForwardCost = {1.4, 0.481, 0.0741};
+// Forward with the pipelined kernel, whose row and column passes overlap: of
+// eleven sets of weights over eight batches of 3 to 24 images, the one with the
+// shortest times (geometric mean 169.3 us; 175.5 with the weights above, up to
+// 13% apart in a batch).
+constexpr TileCost kPipelinedCost = {1.35, 0.70, 0.04};
 // Backward (16 x 512 x 512, residual 11 k of about 300 k cycles an item): 61 k,
 // 19.2 k, 1.68 k of 31.0 k cycles.
 constexpr TileCost kBackwardCost = {1.97, 0.62, 0.0543};

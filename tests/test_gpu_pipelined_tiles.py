@@ -46,15 +46,19 @@ def test_pipelined_maps_equal_phased(monkeypatch, w, h, lam):
         assert np.array_equal(maps[0][s], maps[1][s]), s
 
 
-def test_pipelined_kernel_keeps_its_speed():
+@pytest.mark.parametrize("sizes,scales,plan,bound", [
+    ([(1280, 720), (1920, 1080), (640, 480), (1600, 900)], 8, (0, 0, 0), 1.18),
+    # the split plan, with cost weights of this kernel's own: 1.05 (1.12 with the phased kernel's)
+    ([(58, 444), (680, 636), (45, 839), (55, 119)], 6, (0, 1, 296), 1.09),
+])
+def test_pipelined_kernel_keeps_its_speed(sizes, scales, plan, bound):
     rng = np.random.default_rng(3)
-    sizes = [(1280, 720), (1920, 1080), (640, 480), (1600, 900)]
-    b = api.Batch(sizes, synth.bank(8), kp_capacity=1 << 18)
+    b = api.Batch(sizes, synth.bank(scales), kp_capacity=1 << 18)
     b.load([rng.integers(0, 256, (h, w), dtype=np.uint8) for w, h in sizes])
     ms = {0: [], 1: []}
-    for _ in range(5):
+    for _ in range(7):
         for kernel in (0, 1):
-            b.set_tile_plan(0, 0, 0, kernel)
+            b.set_tile_plan(*plan, kernel)
             b.run()
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             e0.record()
@@ -66,4 +70,4 @@ def test_pipelined_kernel_keeps_its_speed():
     b.close()
     phased, pipelined = np.median(ms[0]), np.median(ms[1])
     print("phased", phased / 4, "pipelined", pipelined / 4, "ms, ratio", pipelined / phased)
-    assert pipelined <= 1.18 * phased
+    assert pipelined <= bound * phased
